@@ -1,11 +1,13 @@
 """The work that is measured when a change is said to make the engine faster.
 
 Each case is one pass of what a user of the engine has it do, through the entry points such a program calls:
-``ModelRunner.step`` (the step function under generation, serving and trace replay) and ``Engine.generate``.  Weights are random: matrices normal(0, 0.02), norm weights around 1, and, as models are commonly
-started, untied embeddings normal(0, 1) and projections into the residual stream divided by sqrt(2 x layers), so that the
-stream carries its tokens through all layers and the rounding of one layer is not multiplied by the next; token ids are uniform.  The sizes are the repository's own: the small 32-bit configuration of its tests, the Qwen3-8B shape of
-its benchmark, the Rogosun shape of its design comparison (dense feed-forwards: which experts a bfloat16 router
-picks hangs on its rounding, so two correct implementations need not agree there), and one generic small model.
+``ModelRunner.step`` (the step function under generation, serving and trace replay) and ``Engine.generate``. Weights
+are random: matrices normal(0, 0.02), norm weights around 1, and, as models are commonly started, untied embeddings
+normal(0, 1) and projections into the residual stream divided by sqrt(2 x layers), so that the stream carries its
+tokens through all layers and the rounding of one layer is not multiplied by the next; token ids are uniform. The
+sizes are the repository's own: the small 32-bit configuration of its tests, the Qwen3-8B shape of its benchmark, the
+Rogosun shape of its design comparison (dense feed-forwards: which experts a bfloat16 router picks hangs on its
+rounding, so two correct implementations need not agree there), and one generic small model.
 
 ``listed()`` gives the named cases, ``draw(rng)`` further ones of the same ranges.  ``prepare`` makes the state a
 program holds before the call, ``run`` is one pass, ``work`` what a pass cannot do without, ``tolerance`` how far two
@@ -190,7 +192,8 @@ def draw(rng) -> dict:
     dtype = rng.choice(["bf16", "fp32"]) if model == "small" else "bf16"
     if kind == "decode":
         requests = between(1, 64)
-        return dict(kind=kind, model=model, dtype=dtype, requests=requests, mean=between(64 if model == "rogosun" else 16, max(80, min(8192, 40000 // requests))))
+        return dict(kind=kind, model=model, dtype=dtype, requests=requests,
+                    mean=between(64 if model == "rogosun" else 16, max(80, min(8192, 40000 // requests))))
     if kind == "mixed":
         return dict(kind=kind, model=model, dtype=dtype, requests=between(1, 32), mean=between(64 if model == "rogosun" else 16, 1000),
                     portion=between(64 if model == "rogosun" else 16, 512))
