@@ -816,3 +816,26 @@ def test_router_gives_a_token_the_same_choice_and_weights_alone_and_in_a_prompt(
     c, ww = o.moe_router(x[3:4], w, corr, top)
     assert torch.equal(c, c_all[3:4]) and torch.equal(ww, w_all[3:4])
     assert o.kernel_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 64, 64), (3, 1027, 260), (4, 4800, 64), (5, 40, 1028), (12, 2400, 132), (16, 12001, 68), (17, 96, 516),
+                                   (32, 2500, 64), (33, 31, 36), (100, 1024, 256), (150, 1300, 72), (70, 4700, 100), (513, 2049, 40), (9, 65, 4)])
+@pytest.mark.parametrize("odt", DTYPES)
+def test_linear_tiles_of_32_bit_operands_give_the_plain_kernels_bits(M, N, K, odt):
+    """Rows on 16-byte boundaries go to tiles chosen by the sizes, others to the plain kernel: one chain of multiply-adds
+    over k per output in both, so the bits are the same."""
+    o = ops()
+    x = rnd(M, K + 4, scale=2.0)
+    w = rnd(N, K + 8, scale=0.1, seed=1)
+    xs, ws = rnd(M, K + 1, seed=2), rnd(N, K + 5, seed=3)      # the same numbers in rows of an odd pitch
+    xs[:, :K], ws[:, :K] = x[:, :K], w[:, :K]
+    out = torch.full((M, N + 3), 7.0, dtype=odt, device=DEV)
+    got = o.linear(x[:, :K], w[:, :K], out=out[:, :N])
+    assert torch.equal(got, o.linear(xs[:, :K], ws[:, :K], out_dtype=odt))
+    assert torch.equal(got, o.linear(x[:, :K], w[:, :K], out_dtype=odt, fresh_weight=True))
+    assert (out[:, N:] == 7.0).all()                            # nothing is written beside the columns
+    want = x[:, :K].double() @ w[:, :K].double().T
+    # K roundings of partial sums no larger than sum |x w|
+    bound = K * 2.0 ** -24 * (x[:, :K].abs().double() @ w[:, :K].abs().double().T) + want.abs() * (2.0 ** -8 if odt == torch.bfloat16 else 0.0) + 1e-30
+    assert ((got.double() - want).abs() <= bound).all()
+    assert o.kernel_status() == 0

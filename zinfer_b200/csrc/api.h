@@ -58,7 +58,7 @@ int zi_qk_norm_rope_store(const void* src, int dtype, int T, int src_stride, con
                           int write_kv, cudaStream_t stream);
 
 int zi_gemm_simt(void* out, int out_dtype, const void* x, int x_dtype, const void* w, int w_dtype, int M, int N,
-                 int K, int ldx, int ldw, int ldo, cudaStream_t stream);
+                 int K, int ldx, int ldw, int ldo, int early_weights, cudaStream_t stream);
 
 // Batched (`batch` products sx/sw/so/sb elements apart) and grouped (per-tile weight group, gathered rows, sizes on
 // the device) forms of the CUDA-core product; epilogue 0: none, 1: square of relu; tile_rows 16 or 64.

@@ -5,6 +5,8 @@
 // order, so a row's result does not depend on which other rows are in the batch.
 #include "api.h"
 #include "common.cuh"
+#include "gemm_f32_tiles.cuh"
+#include "gemm_internal.h"
 
 namespace {
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
@@ -217,14 +219,59 @@ extern "C" int zi_gemm_simt_general(void* out, int out_dtype, const void* x, int
 }
 
 namespace {
+// 32-bit operands whose rows start on 16-byte boundaries: which tile (gemm_f32_tiles.cuh).  The line between the tiles is
+// how many blocks they make: a chain of K multiply-adds per output cannot be split, so a product is as fast as its
+// blocks fill the 148 SMs, and the larger a thread's tile the fewer bytes of shared memory it reads per multiply-add
+// (128 bytes a clock and SM feed 4 x 4 outputs a thread at about a third of the multiply-adds' rate, 8 x 8 at half).
+// Measured, us on one B200 (rows x columns x K; the plain kernel -> the tile taken; every output's bits are the same):
+//   1 x 1024 x 1024  106 -> 6.5      12 x 1024 x 1024  106 -> 10.2    12 x 6144 x 1024  126 -> 14.4   12 x 1024 x 3072  311 -> 26.5
+//   30 x 1024 x 1024  12.8           100 x 1024 x 1024  29            512 x 1024 x 1024  101 -> 43    512 x 6144 x 1024  336 -> 195
+// and with the tile next to the line: 12 x 6144 x 1024 in tiles of 8 columns 20.2, 12 x 32768 x 1024 in tiles of 16 64.6
+// against 61.9 of 32; 100 x 1024 x 1024 in 32 x 32 tiles 40; 512 x 1024 x 3072 in 64 x 64 tiles 342 against 124 of 32 x 32,
+// 512 x 6144 x 1024 in 32 x 32 tiles 230.
+constexpr int SMS = 148;
+template <typename TO>
+int launch_f32(void* out, const float* x, const float* w, int M, int N, int K, int ldx, int ldw, int ldo, int early,
+               cudaStream_t stream) {
+  const long long blocks32 = (long long)((M + 31) / 32) * ((N + 31) / 32), blocks64 = (long long)((M + 63) / 64) * ((N + 63) / 64);
+  if (K % 4 == 0 && (M <= 32 || blocks32 <= SMS)) {
+    int* status = zi_internal_status_word();
+    if (!status) return zi_refuse("gemm: no device memory for the status word");
+#define ZI_FEW(...) return launch_f32_few<F32Few<__VA_ARGS__>, TO>(out, x, w, M, N, K, ldx, ldw, ldo, early, status, stream)
+    if (M <= 4) {
+      if (N < 32 * SMS) ZI_FEW(4, 8, 1, 1, 256, 4, 16);
+      ZI_FEW(4, 32, 2, 1, 128, 4, 8);
+    }
+    if (M <= 16) {
+      if (N <= 16 * SMS) ZI_FEW(16, 8, 2, 2, 256, 3, 8);
+      if (N <= 80 * SMS) ZI_FEW(16, 16, 2, 2, 128, 4, 4);
+      ZI_FEW(16, 32, 4, 2, 128, 3, 4);
+    }
+    if (M <= 32) {
+      if (N <= 16 * SMS) ZI_FEW(32, 8, 2, 2, 128, 4, 4);
+      ZI_FEW(32, 16, 4, 2, 128, 3, 4);
+    }
+    ZI_FEW(32, 16, 4, 4, 128, 3, 4);
+#undef ZI_FEW
+  }
+  if (blocks64 >= 5 * SMS) return launch_f32_tile<F32Tile<64, 64, 8, 8, 32, 3, 2>, TO>(out, x, w, M, N, K, ldx, ldw, ldo, early, stream);
+  return launch_f32_tile<F32Tile<32, 32, 4, 4, 64, 3, 4>, TO>(out, x, w, M, N, K, ldx, ldw, ldo, early, stream);
+}
 }  // namespace
 
+// early_weights: w is not written by a kernel of this step, so that its first rows may be asked for before the wait for
+// the kernels before this one.
 extern "C" int zi_gemm_simt(void* out, int out_dtype, const void* x, int x_dtype, const void* w, int w_dtype, int M,
-                            int N, int K, int ldx, int ldw, int ldo, cudaStream_t stream) {
+                            int N, int K, int ldx, int ldw, int ldo, int early_weights, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return zi_refuse("gemm: K must be positive, got %d", K);
   using bf = __nv_bfloat16;
   const int key = x_dtype * 4 + w_dtype * 2 + out_dtype;
+  // the tiles' grids count rows in blockIdx.y: at most 65,535 blocks of 32
+  if ((key == 0 || key == 1) && ((uintptr_t)x | (uintptr_t)w) % 16 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && M <= 65535 * 32) {
+    if (key == 0) return launch_f32<float>(out, (const float*)x, (const float*)w, M, N, K, ldx, ldw, ldo, early_weights, stream);
+    return launch_f32<bf>(out, (const float*)x, (const float*)w, M, N, K, ldx, ldw, ldo, early_weights, stream);
+  }
   switch (key) {
     case 0: return launch<float, float, float>(out, x, w, M, N, K, ldx, ldw, ldo, stream);
     case 1: return launch<float, float, bf>(out, x, w, M, N, K, ldx, ldw, ldo, stream);

@@ -762,12 +762,12 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
 
     With ``allow_partials`` a product that was split along K may come back as
     :class:`Partials` (its consumer adds the splits) instead of a tensor.  ``fresh_weight``:
-    ``weight`` is no weight but the output of an earlier kernel of this step (the tensor-core kernel
-    otherwise requests its first weight tiles before it waits for the kernels before it).
+    ``weight`` is no weight but the output of an earlier kernel of this step (the tensor-core kernel and the
+    32-bit tiles otherwise request their first weight tiles before they wait for the kernels before them).
 
     bfloat16 operands that meet TMA's alignment rules go to the tcgen05 kernel; float32
     operands (the true 32-bit path), mixed types and unaligned shapes go to the
-    CUDA-core kernel."""
+    CUDA-core kernels."""
     M, K = x.shape
     N, K2 = weight.shape
     _need(K == K2, f"linear: x has {K} columns, weight has {K2}")
@@ -795,7 +795,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     _need(out.stride(1) == 1, "linear: output rows must be dense")
     with _prof.region(f"linear (CUDA cores) N={N} K={K}", lambda: _nb(weight, out) + M * K * x.element_size(), 2 * M * N * K):
         _check(lib().zi_gemm_simt(_ptr(out), _tag(out), _ptr(x), _tag(x), _ptr(weight), _tag(weight), M, N, K,
-                                  x.stride(0), weight.stride(0), out.stride(0), _stream()), "linear")
+                                  x.stride(0), weight.stride(0), out.stride(0), 0 if fresh_weight else 1, _stream()), "linear")
     if relu2:
         _need(out.is_contiguous(), "linear: the square of relu wants dense results")
         relu2_(out)
@@ -818,7 +818,7 @@ def linear_cuda_cores(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional
     out = torch.empty((M, N), dtype=out_dtype or x.dtype, device=x.device)
     with _prof.region(f"linear (CUDA cores) N={N} K={K}", lambda: _nb(weight, out) + M * K * x.element_size(), 2 * M * N * K):
         _check(lib().zi_gemm_simt(_ptr(out), _tag(out), _ptr(x), _tag(x), _ptr(weight), _tag(weight), M, N, K,
-                                  x.stride(0), weight.stride(0), out.stride(0), _stream()), "linear")
+                                  x.stride(0), weight.stride(0), out.stride(0), 0, _stream()), "linear")
     return out
 
 
