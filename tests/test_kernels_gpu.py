@@ -839,3 +839,19 @@ def test_linear_tiles_of_32_bit_operands_give_the_plain_kernels_bits(M, N, K, od
     bound = K * 2.0 ** -24 * (x[:, :K].abs().double() @ w[:, :K].abs().double().T) + want.abs() * (2.0 ** -8 if odt == torch.bfloat16 else 0.0) + 1e-30
     assert ((got.double() - want).abs() <= bound).all()
     assert o.kernel_status() == 0
+
+
+@pytest.mark.parametrize("nq,nkv,d,page,window", [(4, 2, 16, 16, None), (6, 1, 32, 8, None), (3, 3, 64, 16, 40), (8, 2, 128, 32, None),
+                                                  (5, 1, 64, 3, 7), (4, 1, 128, 16, 33), (2, 1, 32, 64, 1), (14, 2, 64, 16, None)])
+def test_exact_attention_for_groups_of_heads_gives_the_plain_kernels_bits(nq, nkv, d, page, window):
+    """Float pages of the usual head sizes go to a kernel that takes the heads of a kv head together; rows of an odd
+    pitch go to the plain one, whose arithmetic it repeats."""
+    for q_lens, ctx_lens in [([1, 37, 2, 1, 19, 16, 17], [70, 0, 15, 0, 48, 33, 300]), ([1] * 5, [0, 31, 32, 200, 63]), ([64], [0])]:
+        args = _paged_case(torch.float32, nq, nkv, d, page, q_lens, ctx_lens)
+        scale = float(1 / np.sqrt(d))
+        got = ops().paged_attention(window=window, scale=scale, **args)
+        q = args["q"]
+        odd = torch.empty(q.shape[0], q.shape[1] + 1, device=DEV)[:, :q.shape[1]]
+        odd.copy_(q)
+        assert torch.equal(got, ops().paged_attention(window=window, scale=scale, **dict(args, q=odd)))
+        torch.testing.assert_close(got, ref.paged_attention(window=window, scale=scale, **args), **tol(torch.float32))
