@@ -533,3 +533,51 @@ def test_small_kernels_against_plain_formulas():
     assert torch.allclose(got.cpu()[:, :nq * d], want[:, :nq * d], rtol=1e-5, atol=1e-6)
     assert torch.allclose(kd.cpu(), kc, rtol=1e-5, atol=1e-6) and torch.allclose(vd.cpu(), vc)
     assert torch.equal(vd.cpu()[1, :, 3], qkv[0, nq * d:].reshape(nkv, d))          # slot 7: the key as projected
+
+
+@gpu
+@pytest.mark.parametrize("D,V,heads,key_heads", [(16, 8, 2, 2), (48, 40, 4, 2), (80, 33, 3, 1), (128, 256, 2, 1)])
+@pytest.mark.parametrize("delta", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_recurrence_in_chunks_against_64_bits_and_the_walk(D, V, heads, key_heads, delta, dtype):
+    """Portions before, at and behind a chunk's edge and single tokens between them, decays from 1 through e^-40 to 0, from
+    states that are not zero: outputs and states in chunks against a loop in 64-bit arithmetic, beside the walk's."""
+    from zinfer_b200 import ops
+
+    gen = torch.Generator(device=DEV).manual_seed(D + V)
+    q_lens, slots = [64, 1, 2, 65, 300, 1, 63, 129, 16], [2, 0, 3, 9, 5, 7, 1, 8, 4]
+    T = sum(q_lens)
+    r = lambda *s: torch.randn(s, generator=gen, device=DEV)
+    wide = r(T, 2 * key_heads * D + heads * V + 5).to(dtype)                    # views of wider rows
+    q, k, v = wide[:, 3:3 + key_heads * D], wide[:, 3 + key_heads * D:3 + 2 * key_heads * D], wide[:, 5 + 2 * key_heads * D:]
+    k.div_(D ** 0.5)
+    decay = torch.sigmoid(3.0 + 2.0 * r(T, heads * D))
+    decay[:, ::7] = 1.0
+    decay[::5, 1::7] = 4e-18
+    decay[::9, 2::7] = 0.0
+    beta = torch.sigmoid(r(T, heads)) if delta else None
+    state0 = 0.3 * r(11, heads, D, V)
+    cu = np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)
+    step = _step(q_lens, slots)
+    step.max_q_len, step.n_dec = max(q_lens), q_lens.count(1)
+    rep = heads // key_heads
+    q64, k64 = ((t.double().view(T, key_heads, D).repeat_interleave(rep, 1)) for t in (q, k))
+    v64, g64 = v.double().view(T, heads, V), decay.double().view(T, heads, D)
+    want, want_state = torch.empty(T, heads, V, dtype=torch.float64, device=DEV), state0.double()
+    for i, slot in enumerate(slots):
+        S = want_state[slot].clone()
+        for t in range(cu[i], cu[i + 1]):
+            S = g64[t].unsqueeze(-1) * S
+            u = v64[t] if beta is None else beta[t].double().unsqueeze(-1) * (v64[t] - torch.einsum("hdv,hd->hv", S, k64[t]))
+            S = S + k64[t].unsqueeze(-1) * u.unsqueeze(-2)
+            want[t] = torch.einsum("hdv,hd->hv", S, 0.5 * q64[t])
+        want_state[slot] = S
+    got = {}
+    for fast in (False, True):
+        state = state0.clone()
+        o = ops.channel_decay_recurrence(q, k, v, decay, beta, 0.5, state, heads, key_heads, D, V, step, fast=fast)
+        assert torch.equal(state[6], state0[6]) and torch.equal(state[10], state0[10])       # other slots untouched
+        got[fast] = [((a.double() - b).norm() / b.norm()).item() for a, b in ((o.view(T, heads, V), want), (state, want_state))]
+    # 2^-22 for the parts' missing products, 2^-24 a rounding: a few of either, as the walk has them
+    assert max(got[True]) < 2e-6, got
+    assert all(c <= 1.5 * w + 2.0 ** -22 for c, w in zip(got[True], got[False])), got

@@ -38,6 +38,7 @@ def lib() -> ctypes.CDLL:
         _LIB.zi_gemm_tcgen05_plan.restype = ctypes.c_longlong
         _LIB.zi_attention_decode_workspace_floats.restype = ctypes.c_longlong
         _LIB.zi_linear_recurrence_tiles_floats.restype = ctypes.c_longlong
+        _LIB.zi_channel_recurrence_workspace_floats.restype = ctypes.c_longlong
         _LIB.zi_chunked_recurrence_workspace_floats.restype = ctypes.c_longlong
     return _LIB
 
@@ -1882,6 +1883,45 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: 
 
 RECURRENCE_CHUNKS = os.environ.get("ZINFER_B200_RECURRENCE_CHUNKS", "1") not in ("", "0")   # off: every request in one walk (comparisons)
 RECURRENCE_CHUNK_MIN = 96     # from this many tokens in a request's portion the chunked form pays
+
+
+def _channel_chunks_pay(longest: int, tokens: int, delta: bool) -> bool:
+    """Whether a step's portions with one decay per key channel run in chunks: the walk takes 0.37 us a token of the longest portion
+    until its blocks fill the GPU, the chunks 40 us (delta rule 60) and 0.06 (0.09) us a token.  Measured at 8 heads of 128 x 256, us
+    (walk, chunks): plain 1 x 96 39.7, 40.3; 1 x 256 98, 45; 8 x 64 107, 66; 4 x 32 31, 43; delta rule 1 x 128 57, 68; 1 x 256 109, 74;
+    8 x 64 120, 102; 4 x 32 35, 70."""
+    return longest >= (160 if delta else 112) or (longest >= 48 and tokens >= 400)
+
+
+def channel_decay_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, beta: Optional[torch.Tensor],
+                             q_scale: float, state: torch.Tensor, heads: int, key_heads: int, dim: int, vdim: int, step, fast: bool) -> torch.Tensor:
+    """The recurrence with one decay per key channel, between 0 and 1 (see :func:`linear_recurrence`; with ``beta`` the delta
+    rule): token by token, or, where ``fast`` allows the tensor cores' products (each operand in two tf32 parts) and a portion is
+    long, in chunks of 64 tokens, single tokens of the same step token by token.  Returns float32 [T, heads * vdim]."""
+    T = q.shape[0]
+    L = lib()
+    delta = beta is not None
+    if not (fast and RECURRENCE_CHUNKS and _channel_chunks_pay(step.max_q_len, T, delta) and L.zi_channel_recurrence_supported(dim, vdim, heads, key_heads)):
+        return linear_recurrence(q, k, v, decay, beta, q_scale, state, heads, key_heads, dim, vdim, step)
+    st, stride = _slot_view(state, "channel_decay_recurrence")
+    _need(st[0].numel() == heads * dim * vdim, "channel_decay_recurrence: state [slots, heads, dim, vdim]")
+    _need(q.dtype == k.dtype and q.stride(1) == 1 and k.stride(1) == 1 and v.stride(1) == 1 and tuple(q.shape) == (T, key_heads * dim)
+          and tuple(k.shape) == (T, key_heads * dim) and tuple(v.shape) == (T, heads * vdim),
+          "channel_decay_recurrence: q, k [T, key heads * dim], v [T, heads * vdim] with dense rows")
+    _need(decay.dtype == torch.float32 and decay.stride(1) == 1 and tuple(decay.shape) == (T, heads * dim), "channel_decay_recurrence: decay")
+    _need(not delta or (beta.dtype == torch.float32 and beta.stride(1) == 1 and tuple(beta.shape) == (T, heads)), "channel_decay_recurrence: beta")
+    out = torch.empty((T, heads * vdim), dtype=torch.float32, device=q.device)
+    n = L.zi_channel_recurrence_workspace_floats(T, step.n_seqs, heads, dim, vdim, 1 if delta else 0)
+    ws = torch.empty((n,), dtype=torch.float32, device=q.device)
+    with _prof.region("recurrence in chunks, decays per channel" + (" (delta rule)" if delta else ""),
+                      lambda: _nb(q, k, v, decay, out) + 2 * step.n_seqs * heads * dim * vdim * 4, 6 * T * heads * dim * vdim):
+        _check(L.zi_channel_recurrence(
+            _ptr(out), out.stride(0), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _tag(q), _ptr(v), v.stride(0), _tag(v), _ptr(decay),
+            decay.stride(0), _ptr(beta), beta.stride(0) if delta else 0, ctypes.c_float(q_scale), _ptr(st), _ll(stride), T, heads, key_heads,
+            dim, vdim, 1 if delta else 0, _ptr(step.cu_q), _ptr(step.state_slots), step.n_seqs, _ptr(ws), _stream()), "channel_recurrence")
+    if step.n_dec > 0:
+        linear_recurrence(q, k, v, decay, beta, q_scale, state, heads, key_heads, dim, vdim, step, only_single=True, out=out)
+    return out
 
 
 def head_decay_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_decay: torch.Tensor, beta: torch.Tensor, state: torch.Tensor,

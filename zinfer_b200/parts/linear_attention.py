@@ -87,8 +87,8 @@ class GatedLinearAttention(Mixer):
         q, k, v, g = proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:2 * qk + hv], proj[:, 2 * qk + hv:2 * qk + 2 * hv]
         z = ops.linear(proj[:, 2 * qk + 2 * hv:], self.w_a2, out_dtype=torch.float32)
         decay = ops.decay_sigmoid_root_(z, self.a_bias, self.tau)
-        o = ops.linear_recurrence(q, k, v, decay, None, self.dim ** -0.5, cache.state, self.heads, self.heads, self.dim,
-                                  self.vdim, step)
+        o = ops.channel_decay_recurrence(q, k, v, decay, None, self.dim ** -0.5, cache.state, self.heads, self.heads, self.dim, self.vdim, step,
+                                         fast=self.ctx.dtype == torch.bfloat16)
         y = ops.head_norm_gate(o, self.norm, self.eps, g, "silu", self.heads, self.vdim, self.ctx.dtype)
         return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
 
@@ -239,7 +239,8 @@ class GatedDeltaRule(Mixer):
         a0 = C + H
         z = ops.linear(proj[:, a0:a0 + self.decay_rank], self.w_a2, out_dtype=torch.float32)
         decay = ops.decay_exp_softplus_(z, self.dt_bias, self.a_log, self.dim)
-        o = ops.linear_recurrence(q, k, v, decay, beta, self.dim ** -0.5, s_view, H, self.kv_heads, self.dim, self.vdim, step)
+        o = ops.channel_decay_recurrence(q, k, v, decay, beta, self.dim ** -0.5, s_view, H, self.kv_heads, self.dim, self.vdim, step,
+                                         fast=self.ctx.dtype == torch.bfloat16)
         gate = ops.linear(proj[:, a0 + self.decay_rank:], self.w_g2, out_dtype=self.ctx.dtype)
         y = ops.head_norm_gate(o, self.norm, self.eps, gate, "sigmoid", H, self.vdim, self.ctx.dtype)
         return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)

@@ -126,7 +126,7 @@ def region(name: str, nbytes=0, flops=0):
 
 # ------------------------------------------------------------------ timeline of a chain
 _TRACE_FILES = ("elementwise", "gemm_tcgen05", "attention_mma", "sampling", "attention_tcgen05", "attention_generic",
-                "gemm_simt")
+                "gemm_simt", "channel_recurrence")
 
 
 def chain_timeline(run_step, warm: int = 2) -> list[dict]:
