@@ -855,3 +855,34 @@ def test_exact_attention_for_groups_of_heads_gives_the_plain_kernels_bits(nq, nk
         odd.copy_(q)
         assert torch.equal(got, ops().paged_attention(window=window, scale=scale, **dict(args, q=odd)))
         torch.testing.assert_close(got, ref.paged_attention(window=window, scale=scale, **args), **tol(torch.float32))
+
+
+@pytest.mark.parametrize("M,N,K", [(130, 4096, 4096), (300, 1024, 12288), (536, 4096, 12288), (257, 2050, 8200), (512, 12288, 512), (1024, 1280, 4160)])
+def test_products_that_the_rule_gives_to_cta_pairs(M, N, K):
+    """More than 128 tokens: the rule between the single-CTA kernel and CTA pairs, with and without a K split, plain, with
+    the square of relu, as partial sums, with fresh weights (which pairs do not take) and gated."""
+    o = ops()
+    x = rnd(M, K, dtype=torch.bfloat16)
+    w = rnd(N, K, dtype=torch.bfloat16, scale=0.05, seed=1)
+    want = x.double() @ w.double().T
+    # K products whose sums are rounded K / 16 times at most, each by 2^-23 of the sum of their sizes (tensor cores round down)
+    bound = K / 16 * 2.0 ** -23 * (x.abs().double() @ w.abs().double().T) + 1e-6
+    got = o.linear(x, w, out_dtype=torch.float32)
+    assert ((got.double() - want).abs() <= bound).all()
+    assert ((o.linear(x, w, out_dtype=torch.float32, fresh_weight=True).double() - want).abs() <= bound).all()
+    half = o.linear(x, w)
+    assert ((half.double() - want).abs() <= bound + 2.0 ** -8 * want.abs()).all()
+    part = o.linear(x, w, allow_partials=True)
+    total = part.sum(torch.float32) if isinstance(part, o.Partials) else part.float()
+    assert ((total.double() - want).abs() <= bound + (0 if isinstance(part, o.Partials) else 2.0 ** -8) * want.abs()).all()
+    sq = o.linear(x, w, out_dtype=torch.float32, relu2=True)
+    top = torch.relu(want)
+    assert ((sq.double() - top ** 2).abs() <= 2 * bound * (top + bound) + bound ** 2 + 2.0 ** -23 * top ** 2).all()
+    if N % 256 == 0:
+        wg, wu = w[:N // 2].contiguous(), w[N // 2:].contiguous()
+        for act in ("silu", "gelu_tanh"):
+            g, u = want[:, :N // 2], want[:, N // 2:]
+            f = g / (1 + torch.exp(-g)) if act == "silu" else torch.nn.functional.gelu(g, approximate="tanh")
+            y = o.linear_swiglu(x, o.interleave_gate_up(wg, wu), activation=act)
+            torch.testing.assert_close(y.double(), f * u, rtol=1.6e-2, atol=2e-3 * K ** 0.5 * 0.05 + 1e-3)
+    assert o.kernel_status() == 0

@@ -108,7 +108,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   uint8_t* v_s = k_s + 2 * TILE_BYTES;       // [2 stages][2 halves of d][128 keys][128 B]
   Barriers* bar = reinterpret_cast<Barriers*>(v_s + 2 * TILE_BYTES);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int h = blockIdx.x, kvh = h / (nq / nkv);
   const int tok0 = cu_q[seq], qlen = cu_q[seq + 1] - tok0, kvlen = kv_lens[seq];
   const int ctx = kvlen - qlen;
@@ -210,17 +210,20 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_max > 0) {
+    if (n_max > 0) {       // the whole warp waits; one elected lane issues
       const uint32_t idesc_s = idesc_bf16(BK, false), idesc_o = idesc_bf16(D, true);
       // S_x[j] = Q_x K[j]^T (K[j] must have arrived: the caller has waited for it)
       auto issue_qk = [&](int x, int j) {
         const uint32_t q_addr = smem_u32(q_s + x * TILE_BYTES), k_addr = smem_u32(k_s + (j & 1) * TILE_BYTES);
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (uint32_t)((kk >> 2) * HALF_BYTES + (kk & 3) * 32);
-          tcgen05_mma_bf16(tmem_s[x], smem_desc_sw128(q_addr + off), smem_desc_sw128(k_addr + off), idesc_s, kk > 0 ? 1u : 0u);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t off = (uint32_t)((kk >> 2) * HALF_BYTES + (kk & 3) * 32);
+            tcgen05_mma_bf16(tmem_s[x], smem_desc_sw128(q_addr + off), smem_desc_sw128(k_addr + off), idesc_s, kk > 0 ? 1u : 0u);
+          }
+          tcgen05_commit(&bar->s_full[x]);
         }
-        tcgen05_commit(&bar->s_full[x]);
+        __syncwarp();
       };
       if (!mbar_wait(&bar->q_full, 0)) { failed = true; atomicExch(status, 14); }
       if (!failed && !mbar_wait(&bar->k_full[0], 0)) { failed = true; atomicExch(status, 12); }
@@ -228,7 +231,8 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         tcgen05_fence_after();
         for (int x = 0; x < 2; ++x)
           if (n_t[x] > 0) issue_qk(x, 0);
-        tcgen05_commit(&bar->k_empty[0]);   // K[0] is free when these products have read it
+        if (elect_one()) tcgen05_commit(&bar->k_empty[0]);   // K[0] is free when these products have read it
+        __syncwarp();
       }
       for (int j = 0; j < n_max && !failed; ++j) {
         const int s = j & 1;
@@ -242,13 +246,16 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           }
           tcgen05_fence_after();
           const uint32_t v_addr = smem_u32(v_s + s * TILE_BYTES);
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            // P: keys kk*16.. = 8 columns of packed pairs; V: key rows kk*16.. of the MN-major V tile
-            umma_bf16_ts(tmem_o[x], tmem_s[x] + (uint32_t)kk * 8u, desc_mnmajor(v_addr + (uint32_t)kk * 16u * 128u), idesc_o,
-                         (j > 0 || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < BK / 16; ++kk) {
+              // P: keys kk*16.. = 8 columns of packed pairs; V: key rows kk*16.. of the MN-major V tile
+              umma_bf16_ts(tmem_o[x], tmem_s[x] + (uint32_t)kk * 8u, desc_mnmajor(v_addr + (uint32_t)kk * 16u * 128u), idesc_o,
+                           (j > 0 || kk > 0) ? 1u : 0u);
+            }
+            tcgen05_commit(&bar->pv_done[x]);
           }
-          tcgen05_commit(&bar->pv_done[x]);
+          __syncwarp();
           if (j + 1 < n_t[x]) {   // the next scores of this tile run under the other tile's softmax
             if (!have_k) {
               if (!mbar_wait(&bar->k_full[(j + 1) & 1], (uint32_t)((j + 1) >> 1) & 1u)) { failed = true; atomicExch(status, 12); break; }
@@ -258,10 +265,11 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             issue_qk(x, j + 1);
           }
         }
-        if (!failed) {
+        if (!failed && elect_one()) {
           tcgen05_commit(&bar->v_empty[s]);                 // V[j] has been read by this iteration's products
           tcgen05_commit(&bar->k_empty[(j + 1) & 1]);       // and K[j+1] by the scores issued in it
         }
+        __syncwarp();
       }
     }
   } else {

@@ -13,7 +13,7 @@
 // Split-K over gridDim.z writes 32-bit partial sums to a workspace; a second kernel
 // adds them in a fixed order.
 //
-// Warp roles (192 threads): warp 0 = TMA producer (a few of its lanes issue side by side), warp 1 = TMEM owner and MMA
+// Warp roles (192 threads): warp 0 = TMA producer, warp 1 = TMEM owner and MMA
 // issuer, warps 2..5 = epilogue (warp w reads TMEM lanes 32*(w%4)..+31).
 // Every wait on an mbarrier is bounded; when it runs out the kernel records a code
 // in `status`, lets copies in flight land, frees its tensor memory and returns.
@@ -91,12 +91,13 @@ __device__ __forceinline__ float gated_mul(float g, float u) {
 // takes part in the warp-wide tensor-memory loads).
 template <typename TO, int EPI>
 __device__ __forceinline__ void drain_accumulator(const GemmArgs& g, TO* __restrict__ out, float* __restrict__ partial,
-                                                  int split, int a, bool a_ok, int b_tile, uint32_t lane_base) {
-  const int BN = g.BN;
+                                                  int split, int a, bool a_ok, int b_tile, uint32_t lane_base, int c_first = 0,
+                                                  int c_end = -1) {
+  const int BN = g.BN, c_stop = c_end < 0 ? BN : c_end;      // columns c_first .. c_stop - 1 of the tile
   constexpr bool SWIGLU = EPI == EPI_SWIGLU || EPI == EPI_GEGLU;
   if (SWIGLU) {
     // Tokens on the lanes; of every 128 columns the first 64 are gate and the next 64 up.
-    for (int c0 = 0; c0 < BN; c0 += 128) {
+    for (int c0 = c_first; c0 < c_stop; c0 += 128) {
 #pragma unroll
       for (int h = 0; h < 64; h += 32) {
         float gv[32], uv[32];
@@ -123,7 +124,7 @@ __device__ __forceinline__ void drain_accumulator(const GemmArgs& g, TO* __restr
       }
     }
   } else
-  for (int c0 = 0; c0 < BN; c0 += 32) {
+  for (int c0 = c_first; c0 < c_stop; c0 += 32) {
     float v[32];
     if (BN - c0 >= 32) {
       tmem_load32(lane_base + (uint32_t)c0, v);
@@ -229,7 +230,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   uint64_t* accum_empty = accum_full + 2;      // [2]
   uint32_t* tmem_slot = (uint32_t*)(accum_empty + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int tiles_per_split = g.a_tiles * g.b_tiles;
   const int total_tiles = tiles_per_split * g.splits;
   const uint32_t tmem_cols = 2u * (uint32_t)g.acc_cols;
@@ -269,11 +270,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   };
 
   if (warp == 0) {
-    // Issuing a tensor copy holds its thread a few hundred nanoseconds while HBM is busy; copies
-    // issued by several lanes in ONE instruction go out side by side.  So the first tile's
-    // prefetch is one instruction over `pre` lanes (twice: weights before the wait for the kernel
-    // before this one, activations after it), and in the loop lane 0 issues the weight's tile and
-    // lane 1 the activations' in the same instruction.
+    // The whole warp walks the k-blocks and one elected lane issues a stage's two tiles.  The first tile's stages
+    // are asked for in two rounds: weights before the wait for the kernel before this one, activations after it.
     if ((int)blockIdx.x < total_tiles) {
       int a_tile, b_tile, split, kb0, n_kb;
       decode(blockIdx.x, a_tile, b_tile, split, kb0, n_kb);
@@ -313,63 +311,68 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                       use_a ? a_row : b_row);
         }
       };
-      if (lane < pre) {
-        mbar_expect_tx(&full[lane], (uint32_t)stage_bytes);
-        issue(1, lane, lane);   // weights do not depend on the kernel before this one
+      for (int i = 0; i < pre; ++i) {      // weights do not depend on the kernel before this one
+        if (elect_one()) {
+          mbar_expect_tx(&full[i], (uint32_t)stage_bytes);
+          issue(1, i, i);
+        }
+        __syncwarp();
       }
       pdl_wait();
-      if (lane < pre) issue(0, lane, lane);
-      // Few tokens: lanes 0 and 1 walk the k-blocks together (both wait for the stage, lane 0 posts the
-      // byte count, then ONE instruction issues both tiles).  Many tokens: the tensor pipe sets the
-      // pace and one lane issuing both tiles in turn is as fast (and measured slightly faster).
-      const int n_issuers = g.a_is_weight ? 2 : 1;
-      if (lane < n_issuers) {
-        uint32_t it = 0;
-        for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
-          decode(tile, a_tile, b_tile, split, kb0, n_kb);
-          for (int i = 0; i < n_kb; ++i, ++it) {
-            if (tile == (int)blockIdx.x && i < pre) continue;   // requested above
-            const int s = it % stages;
-            const uint32_t phase = (it / stages) & 1u;
-            if (!mbar_wait(&empty[s], phase ^ 1u)) { failed = true; atomicExch(status, 1); break; }
-            if (lane == 0) mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
-            if (n_issuers == 2) {
-              issue(lane == 0 ? 1 : 0, s, i);
-            } else {
-              issue(1, s, i);
-              issue(0, s, i);
-            }
+      for (int i = 0; i < pre; ++i) {
+        if (elect_one()) issue(0, i, i);
+        __syncwarp();
+      }
+      int s = pre == stages ? 0 : pre;       // the stage of the next k-block, and the parity its last use left
+      uint32_t parity = pre == stages ? 0u : 1u;
+      for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
+        decode(tile, a_tile, b_tile, split, kb0, n_kb);
+        for (int i = tile == (int)blockIdx.x ? pre : 0; i < n_kb; ++i) {
+          if (!mbar_wait(&empty[s], parity)) { failed = true; atomicExch(status, 1); break; }
+          if (elect_one()) {
+            mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
+            issue(1, s, i);
+            issue(0, s, i);
+          }
+          __syncwarp();
+          if (++s == stages) {
+            s = 0;
+            parity ^= 1u;
           }
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = instr_desc_bf16(TILE_A, BN);
-      uint32_t it = 0, lt = 0;
-      for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x, ++lt) {
-        int a_tile, b_tile, split, kb0, n_kb;
-        decode(tile, a_tile, b_tile, split, kb0, n_kb);
-        const uint32_t acc = lt & 1u, acc_phase = (lt >> 1) & 1u;
-        if (!mbar_wait(&accum_empty[acc], acc_phase ^ 1u)) { failed = true; atomicExch(status, 4); break; }
+    const uint32_t idesc = instr_desc_bf16(TILE_A, BN);
+    const uint64_t a_first = smem_desc_sw128(smem_u32(smem)), b_first = smem_desc_sw128(smem_u32(smem) + A_TILE_BYTES);
+    uint32_t lt = 0, parity = 0;
+    int s = 0;
+    for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x, ++lt) {
+      int a_tile, b_tile, split, kb0, n_kb;
+      decode(tile, a_tile, b_tile, split, kb0, n_kb);
+      const uint32_t acc = lt & 1u, acc_phase = (lt >> 1) & 1u;
+      if (!mbar_wait(&accum_empty[acc], acc_phase ^ 1u)) { failed = true; atomicExch(status, 4); break; }
+      tcgen05_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * (uint32_t)g.acc_cols;
+      for (int i = 0; i < n_kb; ++i) {
+        if (!mbar_wait(&full[s], parity)) { failed = true; atomicExch(status, 2); break; }
         tcgen05_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * (uint32_t)g.acc_cols;
-        for (int i = 0; i < n_kb; ++i, ++it) {
-          const int s = it % stages;
-          const uint32_t phase = (it / stages) & 1u;
-          if (!mbar_wait(&full[s], phase)) { failed = true; atomicExch(status, 2); break; }
-          tcgen05_fence_after();
-          const uint32_t a_addr = smem_u32(smem + (size_t)s * stage_bytes);
-          const uint32_t b_addr = a_addr + A_TILE_BYTES;
+        if (elect_one()) {
+          const uint64_t off = (uint64_t)((uint32_t)(s * stage_bytes) >> 4);     // descriptors count 16 bytes
 #pragma unroll
-          for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-            tcgen05_mma_bf16(d_tmem, smem_desc_sw128(a_addr + k * UMMA_K * 2), smem_desc_sw128(b_addr + k * UMMA_K * 2),
-                             idesc, (i > 0 || k > 0) ? 1u : 0u);
-          }
+          for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
+            tcgen05_mma_bf16(d_tmem, a_first + off + k * UMMA_K * 2 / 16, b_first + off + k * UMMA_K * 2 / 16, idesc,
+                             (i > 0 || k > 0) ? 1u : 0u);
           tcgen05_commit(&empty[s]);  // frees the stage when these MMAs have read it
         }
-        if (!failed) tcgen05_commit(&accum_full[acc]);
+        __syncwarp();
+        if (++s == stages) {
+          s = 0;
+          parity ^= 1u;
+        }
       }
+      if (!failed && elect_one()) tcgen05_commit(&accum_full[acc]);
+      __syncwarp();
     }
   } else {
     const int quarter = warp & 3;  // the TMEM lanes this warp may read
@@ -424,11 +427,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // shared memory goes away while the other may still signal into it.
 constexpr int PAIR_TILE = 256;
 constexpr int PAIR_STAGE_BYTES = A_TILE_BYTES + (PAIR_TILE / 2) * BLOCK_K * 2;
+// Eight epilogue warps, two per quarter of the lanes: a product of one round of tiles ends with a whole drain that
+// nothing hides (256 columns by four warps took about 4 us).
+constexpr int PAIR_EPI_WARPS = 8, PAIR_THREADS = 64 + 32 * PAIR_EPI_WARPS;
 
-template <typename TO, bool SWIGLU>
-__global__ void __launch_bounds__(THREADS)
+template <typename TO, int EPI>
+__global__ void __launch_bounds__(PAIR_THREADS)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                         TO* __restrict__ out, const GemmArgs g, int* __restrict__ status) {
+                         TO* __restrict__ out, float* __restrict__ partial, const GemmArgs g, int* __restrict__ status) {
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -439,10 +445,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   uint64_t* accum_empty = accum_full + 2;      // [2]
   uint32_t* tmem_slot = (uint32_t*)(accum_empty + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-  const int total_tiles = g.a_tiles * g.b_tiles;
+  const int tiles_per_split = g.a_tiles * g.b_tiles, total_tiles = tiles_per_split * g.splits;
   const uint32_t tmem_cols = 2u * (uint32_t)PAIR_TILE;
   bool failed = false;
 
@@ -453,7 +459,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&accum_full[i], 1);
-      mbar_init(&accum_empty[i], 8);   // one arrival per epilogue warp of either CTA
+      mbar_init(&accum_empty[i], 2 * PAIR_EPI_WARPS);   // one arrival per epilogue warp of either CTA
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -469,81 +475,107 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   cluster_sync_all();   // the other CTA's barriers exist before anything signals them
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const int n_kb = g.k_blocks;
+
+  // tile -> (a_tile, b_tile, split, first k-block, number of k-blocks)
+  auto decode = [&](int tile, int& a_tile, int& b_tile, int& split, int& kb0, int& n_kb) {
+    split = tile / tiles_per_split;
+    const int rem = tile - split * tiles_per_split;
+    b_tile = rem / g.a_tiles;
+    a_tile = rem - b_tile * g.a_tiles;
+    kb0 = split * g.k_blocks_per_split;
+    n_kb = min(g.k_blocks, kb0 + g.k_blocks_per_split) - kb0;
+  };
+  int a_tile, b_tile, split, kb0, n_kb;
 
   if (warp == 0) {
     if (pair < total_tiles) {
-      int b_tile = pair / g.a_tiles, a_tile = pair - b_tile * g.a_tiles;
+      decode(pair, a_tile, b_tile, split, kb0, n_kb);
       const int pre = min(stages, n_kb);
       // which: 1 = this CTA's half of the weight rows of k-block i into stage s, 0 = its tokens
       auto issue = [&](int which, int s, int i) {
         uint8_t* dst = smem + (size_t)s * PAIR_STAGE_BYTES;
         const uint32_t bar = cluster_addr_of(&full[s], 0);
         if (which)
-          tma_load_2d_pair(dst + A_TILE_BYTES, &map_b, bar, i * BLOCK_K, b_tile * PAIR_TILE + (int)rank * (PAIR_TILE / 2));
+          tma_load_2d_pair(dst + A_TILE_BYTES, &map_b, bar, (kb0 + i) * BLOCK_K, b_tile * PAIR_TILE + (int)rank * (PAIR_TILE / 2));
         else
-          tma_load_2d_pair(dst, &map_a, bar, i * BLOCK_K, a_tile * PAIR_TILE + (int)rank * TILE_A);
+          tma_load_2d_pair(dst, &map_a, bar, (kb0 + i) * BLOCK_K, a_tile * PAIR_TILE + (int)rank * TILE_A);
       };
-      if (lane < pre) {
-        if (rank == 0) mbar_expect_tx(&full[lane], 2u * (uint32_t)PAIR_STAGE_BYTES);
-        issue(1, lane, lane);   // weights do not depend on the kernel before this one
+      for (int i = 0; i < pre; ++i) {      // weights do not depend on the kernel before this one
+        if (elect_one()) {
+          if (rank == 0) mbar_expect_tx(&full[i], 2u * (uint32_t)PAIR_STAGE_BYTES);
+          issue(1, i, i);
+        }
+        __syncwarp();
       }
       pdl_wait();
-      if (lane < pre) issue(0, lane, lane);
-      if (lane == 0) {
-        uint32_t it = 0;
-        for (int tile = pair; tile < total_tiles && !failed; tile += n_pairs) {
-          b_tile = tile / g.a_tiles;
-          a_tile = tile - b_tile * g.a_tiles;
-          for (int i = 0; i < n_kb; ++i, ++it) {
-            if (tile == pair && i < pre) continue;   // requested above
-            const int s = it % stages;
-            const uint32_t phase = (it / stages) & 1u;
-            if (!mbar_wait(&empty[s], phase ^ 1u)) { failed = true; atomicExch(status, 5); break; }
+      for (int i = 0; i < pre; ++i) {
+        if (elect_one()) issue(0, i, i);
+        __syncwarp();
+      }
+      int s = pre == stages ? 0 : pre;
+      uint32_t parity = pre == stages ? 0u : 1u;
+      for (int tile = pair; tile < total_tiles && !failed; tile += n_pairs) {
+        decode(tile, a_tile, b_tile, split, kb0, n_kb);
+        for (int i = tile == pair ? pre : 0; i < n_kb; ++i) {
+          if (!mbar_wait(&empty[s], parity)) { failed = true; atomicExch(status, 5); break; }
+          if (elect_one()) {
             if (rank == 0) mbar_expect_tx(&full[s], 2u * (uint32_t)PAIR_STAGE_BYTES);
             issue(1, s, i);
             issue(0, s, i);
+          }
+          __syncwarp();
+          if (++s == stages) {
+            s = 0;
+            parity ^= 1u;
           }
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       const uint32_t idesc = instr_desc_bf16(PAIR_TILE, PAIR_TILE);
-      uint32_t it = 0, lt = 0;
+      const uint64_t a_first = smem_desc_sw128(smem_u32(smem)), b_first = smem_desc_sw128(smem_u32(smem) + A_TILE_BYTES);
+      uint32_t lt = 0, parity = 0;
+      int s = 0;
       for (int tile = pair; tile < total_tiles && !failed; tile += n_pairs, ++lt) {
+        decode(tile, a_tile, b_tile, split, kb0, n_kb);
         const uint32_t acc = lt & 1u, acc_phase = (lt >> 1) & 1u;
         if (!mbar_wait(&accum_empty[acc], acc_phase ^ 1u)) { failed = true; atomicExch(status, 8); break; }
         tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + acc * (uint32_t)PAIR_TILE;
-        for (int i = 0; i < n_kb; ++i, ++it) {
-          const int s = it % stages;
-          const uint32_t phase = (it / stages) & 1u;
-          if (!mbar_wait(&full[s], phase)) { failed = true; atomicExch(status, 6); break; }
+        for (int i = 0; i < n_kb; ++i) {
+          if (!mbar_wait(&full[s], parity)) { failed = true; atomicExch(status, 6); break; }
           tcgen05_fence_after();
-          const uint32_t a_addr = smem_u32(smem + (size_t)s * PAIR_STAGE_BYTES);
-          const uint32_t b_addr = a_addr + A_TILE_BYTES;
+          if (elect_one()) {
+            const uint64_t off = (uint64_t)((uint32_t)(s * PAIR_STAGE_BYTES) >> 4);
 #pragma unroll
-          for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-            tcgen05_mma_bf16_pair(d_tmem, smem_desc_sw128(a_addr + k * UMMA_K * 2),
-                                  smem_desc_sw128(b_addr + k * UMMA_K * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
+              tcgen05_mma_bf16_pair(d_tmem, a_first + off + k * UMMA_K * 2 / 16, b_first + off + k * UMMA_K * 2 / 16, idesc,
+                                    (i > 0 || k > 0) ? 1u : 0u);
+            tcgen05_commit_pair(&empty[s], 3);   // frees the stage in both CTAs when these MMAs have read it
           }
-          tcgen05_commit_pair(&empty[s], 3);   // frees the stage in both CTAs when these MMAs have read it
+          __syncwarp();
+          if (++s == stages) {
+            s = 0;
+            parity ^= 1u;
+          }
         }
-        if (!failed) tcgen05_commit_pair(&accum_full[acc], 3);
+        if (!failed && elect_one()) tcgen05_commit_pair(&accum_full[acc], 3);
+        __syncwarp();
       }
     }
   } else {
     const int quarter = warp & 3;  // the TMEM lanes this warp may read
     uint32_t lt = 0;
     for (int tile = pair; tile < total_tiles && !failed; tile += n_pairs, ++lt) {
-      const int b_tile = tile / g.a_tiles, a_tile = tile - b_tile * g.a_tiles;
+      decode(tile, a_tile, b_tile, split, kb0, n_kb);
       const uint32_t acc = lt & 1u, acc_phase = (lt >> 1) & 1u;
       if (!mbar_wait(&accum_full[acc], acc_phase)) { failed = true; atomicExch(status, 7); break; }
       tcgen05_fence_after();
       const int a = a_tile * PAIR_TILE + (int)rank * TILE_A + quarter * 32 + lane;
       const uint32_t lane_base = tmem_base + acc * (uint32_t)PAIR_TILE + ((uint32_t)(quarter * 32) << 16);
-      drain_accumulator<TO, SWIGLU ? EPI_SWIGLU : EPI_PLAIN>(g, out, nullptr, 0, a, a < g.a_rows, b_tile, lane_base);
+      const int half = (warp - 2) >> 2;         // of the columns
+      drain_accumulator<TO, EPI>(g, out, partial, split, a, a < g.a_rows, b_tile, lane_base, half * (PAIR_TILE / 2), (half + 1) * (PAIR_TILE / 2));
       // this accumulator may be overwritten by the MMAs of the tile after next
       tcgen05_fence_before();
       __syncwarp();
@@ -672,9 +704,8 @@ extern "C" int zi_gemm_tcgen05_supported(const void* x, const void* w, int K, in
          encode_fn() != nullptr;
 }
 
-// Size in bytes of the split-K workspace this call needs (0 when it does not split).
-// `plan` receives {swap, BN, splits}.
-extern "C" long long zi_gemm_tcgen05_plan(int M, int N, int K, int sm_count, int* plan) {
+// The plan of the single-CTA kernel, {swap, BN, splits}.
+static void plan_single(int M, int N, int K, int sm_count, int* plan) {
   const int k_blocks = (K + BLOCK_K - 1) / BLOCK_K;
   // Up to 128 tokens the weight's rows take the MMA's 128 lanes and the tokens its columns: every tile
   // is full, where 65..128 tokens on the lanes would fill half of a second row of tiles (measured at
@@ -730,47 +761,89 @@ extern "C" long long zi_gemm_tcgen05_plan(int M, int N, int K, int sm_count, int
   plan[0] = swap;
   plan[1] = BN;
   plan[2] = splits;
-  return splits > 1 ? (long long)splits * M * N * (long long)sizeof(float) : 0;
 }
 
 namespace {
-// Whether the product goes to the kernel for CTA pairs: switched on (zi_gemm_tcgen05_pair_enable, or
-// ZINFER_B200_GEMM_PAIR=1 in the environment), tokens on the lanes, 256-row tiles on both sides, no
-// K split, and few enough padding rows (300 tokens would fill 512 rows of pair tiles but 384 of
-// single tiles).  Off by default: in a prefill step both kernels run at the pace the power limit
-// allows (1.2-1.3 PFLOP/s), so the pair's lighter shared-memory traffic buys nothing there.
-int g_pair_enabled = -1;   // -1: ask the environment
-bool use_pair_kernel(const int* plan, int M) {
-  if (g_pair_enabled < 0) {
+// Which kernel takes products of more than 128 tokens: -1 ask the environment (ZINFER_B200_GEMM_PAIR: 1 always the one for CTA
+// pairs where it can, 0 never), PAIR_AUTO the one that the rule below expects to be faster.
+constexpr int PAIR_NEVER = 0, PAIR_ALWAYS = 1, PAIR_AUTO = 2;
+int g_pair_mode = -1;
+
+// The kernel for CTA pairs, or not, and its K splits.  Time in whole rounds of tiles: a k-block of a single CTA's 128 x 256
+// (or 128 x 128) tile takes 0.37 (0.31) us, of a pair's 256 x 256 tile 0.335 us (measured on full rounds of real weights; with
+// operands from L2 0.32, 0.31 and 0.29).  Splitting K writes the sums as floats and reads them back, about 6 TB/s in L2,
+// and 3 us more; it has to promise 8 us, for the model is no better than that.  Measured, us (single -> pair): 2048 x 24576 x
+// 4096 282 -> 265, 2048 x 4096 x 12288 156 -> 144, 1024 x 4096 x 12288 80 -> 74, 512 x 24576 x 4096 89 -> 80.
+bool plan_pair(int M, int N, int K, int sm_count, int* plan) {
+  if (g_pair_mode < 0) {
     const char* e = getenv("ZINFER_B200_GEMM_PAIR");
-    g_pair_enabled = (e && e[0] == '1') ? 1 : 0;
+    g_pair_mode = e && e[0] == '1' ? PAIR_ALWAYS : (e && e[0] == '0' ? PAIR_NEVER : PAIR_AUTO);
   }
-  if (!g_pair_enabled || plan[0] || plan[1] != PAIR_TILE || plan[2] != 1) return false;
-  const int pair_rows = (M + PAIR_TILE - 1) / PAIR_TILE * PAIR_TILE, single_rows = (M + TILE_A - 1) / TILE_A * TILE_A;
-  return pair_rows == single_rows || M >= 1024;
+  if (g_pair_mode == PAIR_NEVER || plan[0] || N < PAIR_TILE) return false;
+  if (g_pair_mode == PAIR_ALWAYS) {
+    // as far as it wastes little: 300 tokens would fill 512 rows of pair tiles but 384 of single tiles
+    const int pair_rows = (M + PAIR_TILE - 1) / PAIR_TILE * PAIR_TILE, single_rows = (M + TILE_A - 1) / TILE_A * TILE_A;
+    return plan[1] == PAIR_TILE && plan[2] == 1 && (pair_rows == single_rows || M >= 1024);
+  }
+  const int sms = sm_count > 0 ? sm_count : 148, k_blocks = (K + BLOCK_K - 1) / BLOCK_K;
+  auto time = [&](long long tiles, int slots, int splits, double per_kb) {
+    const long long rounds = (tiles * splits + slots - 1) / slots;
+    const double sums = splits > 1 ? 8.0 * splits * M * (double)N / 6e6 + 3.0 : 0.0;
+    return (double)(rounds * ((k_blocks + splits - 1) / splits)) * per_kb + sums;
+  };
+  const long long singles = (long long)((M + TILE_A - 1) / TILE_A) * ((N + plan[1] - 1) / plan[1]);
+  const long long pairs = (long long)((M + PAIR_TILE - 1) / PAIR_TILE) * ((N + PAIR_TILE - 1) / PAIR_TILE);
+  const double single = time(singles, sms, plan[2], plan[1] >= 256 ? 0.37 : 0.31);
+  const double whole = time(pairs, sms / 2, 1, 0.335);
+  double best = whole;
+  int splits = 1;
+  for (int s = 2; s <= 8 && k_blocks / s >= 8; ++s) {
+    const double t = time(pairs, sms / 2, s, 0.335);
+    if (t < best && t < whole - 8.0) {
+      best = t;
+      splits = s;
+    }
+  }
+  if (best >= single) return false;
+  if (splits > 1) {
+    const int kbps = (k_blocks + splits - 1) / splits;
+    splits = (k_blocks + kbps - 1) / kbps;
+  }
+  plan[1] = PAIR_TILE;
+  plan[2] = splits;
+  return true;
 }
+}  // namespace
+
+// Size in bytes of the split-K workspace this call needs (0 when it does not split).
+// `plan` receives {swap, BN, splits}.
+extern "C" long long zi_gemm_tcgen05_plan(int M, int N, int K, int sm_count, int* plan) {
+  plan_single(M, N, K, sm_count, plan);
+  plan_pair(M, N, K, sm_count, plan);
+  return plan[2] > 1 ? (long long)plan[2] * M * N * (long long)sizeof(float) : 0;
+}
+
+namespace {
 // Rows of the B side's copy box.
-int b_box_rows(const int* plan, int M) { return use_pair_kernel(plan, M) ? PAIR_TILE / 2 : plan[1]; }
+int b_box_rows(const int* plan, bool pair) { return pair ? PAIR_TILE / 2 : plan[1]; }
 
 // Launch of the pair kernel: clusters of two CTAs, as many as are resident at once (74 on 148 SMs).
 // Returns -3 when no cluster fits (the caller then has no maps for the single kernel: an error).
-template <typename TO>
-int launch_pair(void* out, const CUtensorMap& map_a, const CUtensorMap& map_b, GemmArgs g, int M, int N, int K,
-                int* status, int swiglu, const char* what, cudaStream_t stream) {
+template <typename TO, int EPI>
+int launch_pair(void* out, const CUtensorMap& map_a, const CUtensorMap& map_b, GemmArgs g, float* partial, int M, int N,
+                int* status, const char* what, cudaStream_t stream) {
   g.a_tiles = (M + PAIR_TILE - 1) / PAIR_TILE;
   g.b_tiles = (N + PAIR_TILE - 1) / PAIR_TILE;
   g.BN = PAIR_TILE;
   g.acc_cols = PAIR_TILE;
-  g.splits = 1;
-  g.k_blocks_per_split = g.k_blocks;
   g.stages = 6;
-  if (g.stages > g.k_blocks) g.stages = g.k_blocks < 2 ? 2 : g.k_blocks;
+  if (g.stages > g.k_blocks_per_split) g.stages = g.k_blocks_per_split < 2 ? 2 : g.k_blocks_per_split;
   const size_t smem = 1024 + (size_t)g.stages * PAIR_STAGE_BYTES + (2 * g.stages + 4) * sizeof(uint64_t) + 16;
-  auto kern = swiglu ? gemm_tcgen05_pair_kernel<TO, true> : gemm_tcgen05_pair_kernel<TO, false>;
+  auto kern = gemm_tcgen05_pair_kernel<TO, EPI>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return zi_refuse("%s: cannot get %zu bytes of shared memory", what, smem);
   cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(THREADS);
+  cfg.blockDim = dim3(PAIR_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -784,12 +857,12 @@ int launch_pair(void* out, const CUtensorMap& map_a, const CUtensorMap& map_b, G
   // clusters resident at once: asked once per device, kernel and number of stages (no allocation here:
   // this path also serves callers that must not allocate)
   static std::mutex mu;
-  static int resident[64][2][2][8];   // 0 = not asked yet, else the answer + 1
+  static int resident[64][8];   // of this instance; 0 = not asked yet, else the answer + 1
   int clusters = 0, dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return zi_refuse("%s: no current device", what);
   {
     std::lock_guard<std::mutex> lock(mu);
-    int& slot = resident[dev][swiglu ? 1 : 0][sizeof(TO) == 2 ? 1 : 0][g.stages];
+    int& slot = resident[dev][g.stages];
     if (slot == 0) {
       cfg.gridDim = dim3(2 * 148);
       cfg.numAttrs = 1;
@@ -803,11 +876,11 @@ int launch_pair(void* out, const CUtensorMap& map_a, const CUtensorMap& map_b, G
     clusters = slot - 1;
   }
   if (clusters <= 0) return zi_refuse("%s: no cluster of two CTAs fits on this GPU", what);
-  const int total_tiles = g.a_tiles * g.b_tiles;
+  const int total_tiles = g.a_tiles * g.b_tiles * g.splits;
   if (clusters > total_tiles) clusters = total_tiles;
   cfg.gridDim = dim3(2 * clusters);
   cfg.numAttrs = g_zi_pdl_enabled ? 2 : 1;
-  e = cudaLaunchKernelEx(&cfg, kern, map_a, map_b, (TO*)out, g, status);
+  e = cudaLaunchKernelEx(&cfg, kern, map_a, map_b, (TO*)out, partial, g, status);
   if (e != cudaSuccess) return zi_refuse("%s: launch failed: %s", what, cudaGetErrorString(e));
   return zi_check_launch(what);
 }
@@ -844,7 +917,7 @@ int launch_gemm(void* out, int out_dtype, const CUtensorMap& map_a, const CUtens
                 int ldo, const int* plan, float* partial_buf, int* status, int sm_count, int defer_reduce,
                 const char* what, cudaStream_t stream, int epi = EPI_PLAIN, float* cand_val = nullptr,
                 int* cand_idx = nullptr, const int* tile_group = nullptr, int relu2 = 0, int act = ZI_ACT_SILU,
-                int head_groups = 0, int a_group_cols = 0, long long out_group_stride = 0) {
+                int head_groups = 0, int a_group_cols = 0, long long out_group_stride = 0, bool pair = false) {
   const int swap = plan[0], BN = plan[1], splits = plan[2];
   const int swiglu = epi == EPI_SWIGLU;
   const bool geglu = swiglu && act == ZI_ACT_GELU_TANH;
@@ -899,9 +972,7 @@ int launch_gemm(void* out, int out_dtype, const CUtensorMap& map_a, const CUtens
     return zi_refuse("%s: the square of relu goes with the plain product whose splits are added here", what);
   // a split product's partial sums are squared where they are added, an unsplit one's in the epilogue
   const int relu2_epi = relu2 && g.splits == 1, relu2_sum = relu2 && g.splits > 1;
-  if (!tile_group && !head_groups && !geglu && !relu2 && use_pair_kernel(plan, M)) {
-    ZI_DISPATCH_DTYPE(out_dtype, TO, { return launch_pair<TO>(out, map_a, map_b, g, M, N, K, status, swiglu, what, stream); });
-  }
+  if (pair && (tile_group || head_groups || g.late_weights || epi == EPI_ARGMAX)) return zi_refuse("%s: not a product for CTA pairs", what);
   if (epi == EPI_ARGMAX) {
     if (out_dtype != ZI_F32 || !swap || g.splits != 1 || !cand_val || !cand_idx)
       return zi_refuse("%s: the argmax epilogue takes 32-bit results of an unsplit product of at most 128 tokens", what);
@@ -910,7 +981,11 @@ int launch_gemm(void* out, int out_dtype, const CUtensorMap& map_a, const CUtens
   ZI_DISPATCH_DTYPE(out_dtype, TO, {
     const bool ext = g.tile_group || g.late_weights || g.group_tiles;
     const GemmArgs& plain = g;      // the plain product takes its own arguments only
-    int rc = relu2_epi ? launch_single<TO, EPI_RELU2, GemmExtArgs>(out, map_a, map_b, g, partial, status, sm_count, smem, total_tiles, what, stream)
+    int rc = pair ? (relu2_epi ? launch_pair<TO, EPI_RELU2>(out, map_a, map_b, plain, partial, M, N, status, what, stream)
+                     : geglu   ? launch_pair<TO, EPI_GEGLU>(out, map_a, map_b, plain, partial, M, N, status, what, stream)
+                     : swiglu  ? launch_pair<TO, EPI_SWIGLU>(out, map_a, map_b, plain, partial, M, N, status, what, stream)
+                               : launch_pair<TO, EPI_PLAIN>(out, map_a, map_b, plain, partial, M, N, status, what, stream))
+           : relu2_epi ? launch_single<TO, EPI_RELU2, GemmExtArgs>(out, map_a, map_b, g, partial, status, sm_count, smem, total_tiles, what, stream)
            : (ext && !swiglu) ? launch_single<TO, EPI_PLAIN, GemmExtArgs>(out, map_a, map_b, g, partial, status, sm_count, smem, total_tiles, what, stream)
            : geglu ? launch_single<TO, EPI_GEGLU, GemmArgs>(out, map_a, map_b, plain, partial, status, sm_count, smem, total_tiles, what, stream)
            : swiglu ? launch_single<TO, EPI_SWIGLU, GemmArgs>(out, map_a, map_b, plain, partial, status, sm_count, smem, total_tiles, what, stream)
@@ -940,18 +1015,22 @@ extern "C" int zi_gemm_tcgen05(void* out, int out_dtype, const void* x, const vo
   if (!zi_gemm_tcgen05_supported(x, w, K, ldx, ldw))
     return zi_refuse("gemm_tcgen05: operands must be 16-byte aligned bfloat16 with row pitches in multiples of 8");
   int plan[3];
-  const long long need = zi_gemm_tcgen05_plan(M, N, K, sm_count, plan);
+  plan_single(M, N, K, sm_count, plan);
+  // (the kernel for pairs asks for its first weight tiles before the wait for the kernels before it; where `w` is written by one
+  // of them the sums' splits are still the plan's)
+  const bool pair = plan_pair(M, N, K, sm_count, plan) && !((defer_reduce >> 1) & 1);
+  const long long need = plan[2] > 1 ? (long long)plan[2] * M * N * (long long)sizeof(float) : 0;
   if (need > workspace_bytes) return zi_refuse("gemm_tcgen05: split-K needs %lld workspace bytes, got %lld", need, workspace_bytes);
   const int swap = plan[0];
   const int a_rows = swap ? N : M, b_rows = swap ? M : N;
   CUtensorMap map_a, map_b;
   if (!make_map(&map_a, swap ? w : x, a_rows, K, swap ? ldw : ldx, TILE_A) ||
-      !make_map(&map_b, swap ? x : w, b_rows, K, swap ? ldx : ldw, b_box_rows(plan, M)))
+      !make_map(&map_b, swap ? x : w, b_rows, K, swap ? ldx : ldw, b_box_rows(plan, pair)))
     return zi_refuse("gemm_tcgen05: cuTensorMapEncodeTiled failed");
   int* status = status_word();
   if (!status) return zi_refuse("gemm_tcgen05: cannot allocate the status word");
   return launch_gemm(out, out_dtype, map_a, map_b, M, N, K, ldo, plan, workspace, status, sm_count, defer_reduce,
-                     "gemm_tcgen05", stream);
+                     "gemm_tcgen05", stream, EPI_PLAIN, nullptr, nullptr, nullptr, 0, ZI_ACT_SILU, 0, 0, 0, pair);
 }
 
 // Grouped product for a mixture of experts: row r of x [rows, K] (rows a multiple of 128, already laid
@@ -1017,7 +1096,8 @@ extern "C" int zi_gemm_tcgen05_gated(void* out, int out_dtype, const void* x, co
   if (!zi_gemm_tcgen05_supported(x, w, K, ldx, ldw))
     return zi_refuse("gemm_swiglu: operands must be 16-byte aligned bfloat16 with row pitches in multiples of 8");
   int plan[3];
-  zi_gemm_tcgen05_plan(M, N2, K, sm_count, plan);
+  plan_single(M, N2, K, sm_count, plan);
+  const bool pair = plan_pair(M, N2, K, sm_count, plan);
   if (plan[2] > 1) return -2;
   const int swap = plan[0];
   // Few tokens: the separate SwiGLU kernel is the better schedule.  While it runs, the CTAs of
@@ -1028,12 +1108,12 @@ extern "C" int zi_gemm_tcgen05_gated(void* out, int out_dtype, const void* x, co
   const int a_rows = swap ? N2 : M, b_rows = swap ? M : N2;
   CUtensorMap map_a, map_b;
   if (!make_map(&map_a, swap ? w : x, a_rows, K, swap ? ldw : ldx, TILE_A) ||
-      !make_map(&map_b, swap ? x : w, b_rows, K, swap ? ldx : ldw, b_box_rows(plan, M)))
+      !make_map(&map_b, swap ? x : w, b_rows, K, swap ? ldx : ldw, b_box_rows(plan, pair)))
     return zi_refuse("gemm_swiglu: cuTensorMapEncodeTiled failed");
   int* status = status_word();
   if (!status) return zi_refuse("gemm_swiglu: cannot allocate the status word");
   return launch_gemm(out, out_dtype, map_a, map_b, M, N2, K, ldo, plan, nullptr, status, sm_count, 0, "gemm_swiglu",
-                     stream, EPI_SWIGLU, nullptr, nullptr, nullptr, 0, act);
+                     stream, EPI_SWIGLU, nullptr, nullptr, nullptr, 0, act, 0, 0, 0, pair);
 }
 
 // Rows of candidates per token that zi_gemm_tcgen05_argmax leaves: one per 32 weight rows,
@@ -1063,11 +1143,11 @@ extern "C" int zi_gemm_tcgen05_argmax(float* out, const void* x, const void* w, 
                      EPI_ARGMAX, cand_val, cand_idx);
 }
 
-// Switches the kernel for CTA pairs on (1) or off (0) for products of 256 tokens and more; returns
-// the setting before.
+// Switches the kernel for CTA pairs on (1) for products of 256 tokens and more that fill its tiles, or back to the rule
+// that chooses (0); returns the setting before.
 extern "C" int zi_gemm_tcgen05_pair_enable(int on) {
-  const int before = g_pair_enabled > 0 ? 1 : 0;
-  g_pair_enabled = on ? 1 : 0;
+  const int before = g_pair_mode == PAIR_ALWAYS ? 1 : 0;
+  g_pair_mode = on ? PAIR_ALWAYS : PAIR_AUTO;
   return before;
 }
 
@@ -1182,7 +1262,8 @@ extern "C" int zi_gemm_tcgen05_static_scratch(void* out, int out_dtype, const vo
   if (!zi_gemm_tcgen05_supported(x, w, K, ldx, ldw))
     return zi_refuse("gemm_static_scratch: operands must be 16-byte aligned bfloat16 with row pitches in multiples of 8");
   int plan[3];
-  const long long need = zi_gemm_tcgen05_plan(M, N, K, sm_count, plan);
+  plan_single(M, N, K, sm_count, plan);       // the kernel for pairs may split further than the scratch holds
+  const long long need = plan[2] > 1 ? (long long)plan[2] * M * N * (long long)sizeof(float) : 0;
   if (need > zi_gemm_static_scratch_capacity_bytes())
     return zi_refuse("gemm_static_scratch: this product splits K and needs %lld bytes of scratch; the built-in scratch "
                      "holds %lld (use zi_gemm_tcgen05 with a workspace of your own)",
@@ -1196,7 +1277,7 @@ extern "C" int zi_gemm_tcgen05_static_scratch(void* out, int out_dtype, const vo
   const int lda = swap ? ldw : ldx, ldb = swap ? ldx : ldw;
   CUtensorMap map_a, map_b;
   if (!encode_map_direct(&map_a, swap ? w : x, a_rows, K, lda, TILE_A) ||
-      !encode_map_direct(&map_b, swap ? x : w, b_rows, K, ldb, b_box_rows(plan, M)))
+      !encode_map_direct(&map_b, swap ? x : w, b_rows, K, ldb, b_box_rows(plan, false)))
     return zi_refuse("gemm_static_scratch: cuTensorMapEncodeTiled failed");
   // The status word is only ever written with a non-zero code, never cleared here: a failure of an
   // earlier call stays visible until it is read.  The partial sums need no clearing either, every

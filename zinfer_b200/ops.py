@@ -67,10 +67,9 @@ def selftest_wait_runs_out(code: int = 77, tries: int = 4096) -> None:
 
 def gemm_pair_kernel(on: bool) -> bool:
     """Switches the matrix product's kernel for CTA pairs (tcgen05 ``cta_group::2``: two SMs on one
-    tile of 256 tokens x 256 weight rows, each loading half of the weight rows) on or off for
-    products of 256 tokens and more; returns the setting before.  Off unless
-    ``ZINFER_B200_GEMM_PAIR=1``: measured equal to the single-CTA kernel inside a prefill step,
-    where both run at the pace the power limit allows."""
+    tile of 256 tokens x 256 weight rows, each loading half of the weight rows) on for all products of
+    256 tokens and more that fill its tiles, or back to the rule that chooses between the kernels
+    (``ZINFER_B200_GEMM_PAIR``: 1 as here, 0 never, else the rule); returns the setting before."""
     return bool(lib().zi_gemm_tcgen05_pair_enable(1 if on else 0))
 
 
