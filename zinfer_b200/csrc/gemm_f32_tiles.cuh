@@ -22,9 +22,62 @@ struct F32Tile {
   static constexpr size_t SMEM = (size_t)STAGES * STAGE * sizeof(float);
 };
 
+// One 16-byte piece along k of a thread's rows of both operands, and its multiply-adds.
+template <int TM, int TN>
+struct F32Piece {
+  float4 a[TM], b[TN];
+  template <int GAP_A, int GAP_B>
+  __device__ __forceinline__ void read(const float* xs, const float* ws, int p) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(xs + i * GAP_A + p * 4);
+#pragma unroll
+    for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(ws + j * GAP_B + p * 4);
+  }
+  __device__ __forceinline__ void multiply(float (&acc)[TM][TN]) const {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+  }
+};
+
+// A chunk's pieces (all PIECES of it, or fewer at the end of K) in turn, each read one ahead of its use: a warp or two a
+// scheduler cannot hide the reads otherwise (5 % at 12 x 1024 x 1024, 4 % at 512 x 6144 x 1024).
+template <int TM, int TN, int GAP_A, int GAP_B, int PIECES, int UNROLL>
+__device__ __forceinline__ void f32_chunk(float (&acc)[TM][TN], const float* xs, const float* ws, int pieces) {
+  F32Piece<TM, TN> even, odd;
+  if (pieces == PIECES) {
+    even.template read<GAP_A, GAP_B>(xs, ws, 0);
+#pragma unroll UNROLL
+    for (int p = 0; p < PIECES; p += 2) {
+      odd.template read<GAP_A, GAP_B>(xs, ws, p + 1);
+      even.multiply(acc);
+      if (p + 2 < PIECES) even.template read<GAP_A, GAP_B>(xs, ws, p + 2);
+      odd.multiply(acc);
+    }
+  } else {
+    for (int p = 0; p < pieces; ++p) {
+      even.template read<GAP_A, GAP_B>(xs, ws, p);
+      even.multiply(acc);
+    }
+  }
+}
+
 // Bound by shared memory: a 16-byte read by a warp takes four of the SM's 128-byte clocks whatever the addresses, so the
 // plain kernel's one-word reads left the multiply-adds idle most of the time (512 x 6144 x 1024: 336 us, 19 TFLOP/s; now
-// 195 us, 33, of the 69 that independent chains of fmaf reach here).  A ring of STAGES chunks of KC columns, filled by cp.async; a thread owns TM x TN outputs, rows BM / TM and columns
+// 187 us, 34, of the 69 that independent chains of fmaf reach here).  A ring of STAGES chunks of KC columns, filled by cp.async; a thread owns TM x TN outputs, rows BM / TM and columns
 // BN / TN apart, and reads both operands as 16-byte pieces along k.  `early`: w is not written by a kernel of this
 // step, so its first chunks are requested before the wait for the kernels before this one.
 template <typename T, typename TO>
@@ -77,31 +130,7 @@ gemm_f32_tile_kernel(TO* __restrict__ out, const float* __restrict__ x, const fl
     asm volatile("cp.async.commit_group;" ::: "memory");
     const float* xs = f32_smem + (c % STAGES) * T::STAGE + ty * PITCH;
     const float* ws = f32_smem + (c % STAGES) * T::STAGE + (BM + tx) * PITCH;
-    const int pieces = (min(KC, K - c * KC) + 3) / 4;
-#pragma unroll T::UNROLL
-    for (int p = 0; p < pieces; ++p) {
-      float4 a[TM], b[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(xs + i * ROWS_M * PITCH + p * 4);
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(ws + j * ROWS_N * PITCH + p * 4);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
-    }
+    f32_chunk<TM, TN, ROWS_M * PITCH, ROWS_N * PITCH, PIECES, T::UNROLL>(acc, xs, ws, (min(KC, K - c * KC) + 3) / 4);
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -131,8 +160,9 @@ int launch_f32_tile(void* out, const float* x, const float* w, int M, int N, int
 // Up to 32 rows: the same tiles with a warp of their own for the copies.  One lane per operand row asks for KC columns of
 // it in one untiled bulk copy (both ends on 16-byte boundaries, sizes of whole 16 bytes: K % 4 == 0), so the warps that
 // multiply issue nothing but shared-memory reads and multiply-adds.  Bound by the chain itself: K dependent multiply-adds of
-// four clocks and the reads that feed them (12 x 1024 x 1024: 10.2 us, 4 MB of weights; 18 us with copies by the same warps,
-// whose addresses cost more issue slots than the product).
+// four clocks and the reads that feed them (12 x 1024 x 1024: 9.5 us, 4 MB of weights; 18 us with copies by the same warps,
+// whose addresses cost more issue slots than the product).  One tensor copy a chunk in the place of one bulk copy a row,
+// its lines swizzled, was measured too: 11.1 us, for the addresses of the swizzled reads.
 template <int BM_, int BN_, int TM_, int TN_, int KC_, int STAGES_, int UNROLL_>
 struct F32Few {
   static constexpr int BM = BM_, BN = BN_, TM = TM_, TN = TN_, KC = KC_, STAGES = STAGES_, UNROLL = UNROLL_;
@@ -217,29 +247,6 @@ gemm_f32_few_kernel(TO* __restrict__ out, const float* __restrict__ x, const flo
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-  auto multiply = [&](const float* xs, const float* ws, int p) {
-    float4 a[TM], b[TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(xs + i * ROWS_M * PITCH + p * 4);
-#pragma unroll
-    for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(ws + j * ROWS_N * PITCH + p * 4);
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
-  };
   for (int c = 0; c < chunks; ++c) {
     const int s = c % STAGES;
     if (!mbar_wait(&full[s], (c / STAGES) & 1)) {
@@ -248,13 +255,7 @@ gemm_f32_few_kernel(TO* __restrict__ out, const float* __restrict__ x, const flo
     }
     const float* xs = f32_smem + (size_t)s * T::STAGE + ty * PITCH;
     const float* ws = f32_smem + (size_t)s * T::STAGE + (BM + tx) * PITCH;
-    const int pieces = min(KC, K - c * KC) / 4;
-    if (pieces == KC / 4) {
-#pragma unroll T::UNROLL
-      for (int p = 0; p < KC / 4; ++p) multiply(xs, ws, p);
-    } else {
-      for (int p = 0; p < pieces; ++p) multiply(xs, ws, p);
-    }
+    f32_chunk<TM, TN, ROWS_M * PITCH, ROWS_N * PITCH, KC / 4, T::UNROLL>(acc, xs, ws, min(KC, K - c * KC) / 4);
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);
   }
