@@ -135,3 +135,32 @@ def test_a_token_in_a_page_already_given_back_is_refused():
     m.reserve("a", 1)
     ctx = build_step(m, [StepEntry("a", [5], [0])], "cpu", tile_rows=8, pin=False)
     assert ctx.kv_groups[0].block_tables[0].tolist()[0] == -1 and ctx.kv_groups[0].slot_mapping.tolist()[0] >= 0
+
+
+def test_a_bucket_is_refilled_as_it_is_built():
+    """Further steps of a bucket write the same arrays into the same places as a build from nothing: requests that have
+    grown, fewer of them, tokens taken from the step before."""
+    from zinfer_b200.engine.batch import refill_static
+
+    m = _manager()
+    for rid, n in (("a", 5), ("b", 1), ("c", 9)):
+        m.add_request(rid)
+        m.reserve(rid, n)
+        m.commit(rid, n)
+    statics = [StaticStepBuffers(4, 5, "cpu", max_kv_len=20) for _ in range(2)]
+    first = [StepEntry("a", [3], [0]), StepEntry("b", [4], [0]), StepEntry("c", [5], [])]
+    for rid in "abc":
+        m.reserve(rid, 1)
+    for s in statics:
+        build_step(m, first, "cpu", tile_rows=8, static=s, pf_tile_rows=16)
+    for rid in "abc":
+        m.commit(rid, 1)
+    for entries in ([StepEntry("c", [6], [0]), StepEntry("a", [7], [0])], [StepEntry("b", [-1], [0], token_src=2)],
+                    [StepEntry("a", [1], []), StepEntry("b", [-1], [0], token_src=0), StepEntry("c", [2], [0])]):
+        for e in entries:
+            m.reserve(e.request_id, 1)
+        ctx = build_step(m, entries, "cpu", tile_rows=8, static=statics[0], pf_tile_rows=16)
+        assert refill_static(m, entries, statics[1], 8, 16) == ctx.n_patch
+        assert torch.equal(statics[1].device_buffer(statics[1].total), statics[0].device_buffer(statics[0].total))
+        for e in entries:
+            m.commit(e.request_id, 1)

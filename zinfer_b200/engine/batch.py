@@ -181,6 +181,28 @@ def build_step(manager: CacheManager, entries: Sequence[StepEntry], device, tile
         all_decode=all(q == 1 for q in q_lens), h2d_bytes=int(total) * 4)
 
 
+def refill_static(manager: CacheManager, entries: Sequence[StepEntry], static: "StaticStepBuffers", tile_rows: int,
+                  pf_tile_rows: int) -> int:
+    """The arrays of a further step of a bucket that :func:`build_step` has built one for: the same places and sizes, new
+    contents, copied to the device.  What replays a captured graph needs no views of them.  Returns the number of tokens
+    to be taken from the step before."""
+    n = len(entries)
+    ids, ones, tokens, wants, zeros, src, layout = static.words(2 * (len(_ARRAYS) + 2 * len(manager.groups)) + 10 + len(manager.groups))
+    ids[:n] = [manager.native_id(e.request_id) for e in entries]
+    tokens[:n] = [e.tokens[0] for e in entries]
+    wants[:n] = [len(e.want) for e in entries]
+    src[:n] = [-1 if e.token_src is None else e.token_src for e in entries]
+    hostbuf = static.host_buffer(static.total)
+    total = host.lib().zi_step_build(manager.handle, n, ids.ctypes.data, ones.ctypes.data, tokens.ctypes.data, wants.ctypes.data,
+                                     zeros.ctypes.data, src.ctypes.data, static.batch, static.width, tile_rows, pf_tile_rows,
+                                     hostbuf.data_ptr(), static.total, layout.ctypes.data)
+    if total < 0:
+        raise RuntimeError(f"the step cannot be built: {host.last_error()}")
+    static.device_buffer(static.total).copy_(hostbuf, non_blocking=True)
+    static.mark_copied()
+    return int(layout[2 * (len(_ARRAYS) + 2 * len(manager.groups)) + 7])
+
+
 class StaticStepBuffers:
     """Pinned host and device buffers of fixed address for the decode steps of one
     batch-size bucket, so that a captured CUDA graph finds every step's arrays at the
@@ -194,6 +216,20 @@ class StaticStepBuffers:
         self._host = None
         self._dev = None
         self._copied = None
+        self._words = None
+
+    @property
+    def total(self) -> int:
+        """The arrays' size in 32-bit words, known once a step has been built here."""
+        return self._host.numel()
+
+    def words(self, n_layout: int) -> tuple:
+        """What the native builder reads and the layout it leaves, as arrays that steps reuse: requests, tokens each (one),
+        tokens, wanted places each, wanted places (0), rows of the step before, layout."""
+        if self._words is None:
+            i32 = lambda v: np.full(self.batch, v, dtype=np.int32)
+            self._words = (np.zeros(self.batch, dtype=np.int64), i32(1), i32(0), i32(0), i32(0), i32(-1), np.zeros(n_layout, dtype=np.int64))
+        return self._words
 
     def host_buffer(self, total: int) -> torch.Tensor:
         """The pinned staging buffer, safe to overwrite: the copy of the previous

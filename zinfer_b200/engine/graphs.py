@@ -24,7 +24,7 @@ from typing import Optional, Sequence
 import torch
 
 from .. import ops
-from .batch import StaticStepBuffers, StepEntry, build_step
+from .batch import StaticStepBuffers, StepEntry, build_step, refill_static
 
 BUCKETS = (1, 2, 4, 8, 16, 24, 32, 48, 64, 96, 128, 192, 256)
 MIN_CONTEXT_BUCKET = 256
@@ -75,30 +75,37 @@ class DecodeGraphs:
             static = StaticStepBuffers(b, -(-ctx_bucket // ps), runner.device, max_kv_len=ctx_bucket)
             state = self._buckets[key] = {"static": static, "graph": None, "outputs": None, "launches": 0, "warm": 0}
         self._buckets.move_to_end(key)
+        if state["graph"] is not None:       # captured: the arrays alone are new
+            token_ids, patch_dst, patch_src, runner.last_h2d_bytes = state["arrays"]
+            if refill_static(runner.manager, entries, state["static"], runner.tile_rows, runner.pf_tile_rows):
+                ops.patch_tokens(token_ids, prev_tokens, patch_dst, patch_src)
+            return self._replay(state)
         ctx = build_step(runner.manager, entries, runner.device, runner.tile_rows, static=state["static"],
                          pf_tile_rows=runner.pf_tile_rows)
         runner.last_h2d_bytes = ctx.h2d_bytes
         if ctx.n_patch:   # outside the graph: which rows are patched changes from step to step
             ops.patch_tokens(ctx.token_ids, prev_tokens, ctx.patch_dst, ctx.patch_src)
-        if state["graph"] is None:
-            if state["warm"] < 1:
-                # first use: run uncaptured, so that one-time set-up (function attributes,
-                # rotary tables, the kernels' status word) happens outside a capture
-                state["warm"] += 1
-                return runner.model.forward(ctx, argmax=True)
-            torch.cuda.synchronize()
-            graph = torch.cuda.CUDAGraph()
-            before = ops.LAUNCHES
-            # relaxed: a host-side call that touches no captured work (the pinned-memory allocator
-            # polling an old event when Python frees a buffer) must not invalidate the capture
-            if self._pool is None:
-                self._pool = torch.cuda.graph_pool_handle()
-            with torch.cuda.graph(graph, pool=self._pool, capture_error_mode="relaxed"):
-                state["outputs"] = runner.model.forward(ctx, argmax=True)
-            self.captures += 1
-            state["launches"] = ops.LAUNCHES - before
-            ops.LAUNCHES = before
-            state["graph"] = graph
+        if state["warm"] < 1:
+            # first use: run uncaptured, so that one-time set-up (function attributes,
+            # rotary tables, the kernels' status word) happens outside a capture
+            state["warm"] += 1
+            return runner.model.forward(ctx, argmax=True)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        before = ops.LAUNCHES
+        # relaxed: a host-side call that touches no captured work (the pinned-memory allocator
+        # polling an old event when Python frees a buffer) must not invalidate the capture
+        if self._pool is None:
+            self._pool = torch.cuda.graph_pool_handle()
+        with torch.cuda.graph(graph, pool=self._pool, capture_error_mode="relaxed"):
+            state["outputs"] = runner.model.forward(ctx, argmax=True)
+        self.captures += 1
+        state["launches"] = ops.LAUNCHES - before
+        ops.LAUNCHES = before
+        state["graph"], state["arrays"] = graph, (ctx.token_ids, ctx.patch_dst, ctx.patch_src, ctx.h2d_bytes)
+        return self._replay(state)
+
+    def _replay(self, state: dict):
         state["graph"].replay()
         self.replays += 1
         self.launches += state["launches"]
