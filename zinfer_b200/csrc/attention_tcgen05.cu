@@ -225,8 +225,8 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         }
         __syncwarp();
       };
-      if (!mbar_wait(&bar->q_full, 0)) { failed = true; atomicExch(status, 14); }
-      if (!failed && !mbar_wait(&bar->k_full[0], 0)) { failed = true; atomicExch(status, 12); }
+      if (!warp_mbar_wait(&bar->q_full, 0)) { failed = true; atomicExch(status, 14); }
+      if (!failed && !warp_mbar_wait(&bar->k_full[0], 0)) { failed = true; atomicExch(status, 12); }
       if (!failed) {
         tcgen05_fence_after();
         for (int x = 0; x < 2; ++x)
@@ -239,9 +239,9 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         bool have_v = false, have_k = false;
         for (int x = 0; x < 2 && !failed; ++x) {
           if (j >= n_t[x]) continue;
-          if (!mbar_wait(&bar->p_full[x], (uint32_t)j & 1u)) { failed = true; atomicExch(status, 15); break; }
+          if (!warp_mbar_wait(&bar->p_full[x], (uint32_t)j & 1u)) { failed = true; atomicExch(status, 15); break; }
           if (!have_v) {
-            if (!mbar_wait(&bar->v_full[s], (uint32_t)(j >> 1) & 1u)) { failed = true; atomicExch(status, 16); break; }
+            if (!warp_mbar_wait(&bar->v_full[s], (uint32_t)(j >> 1) & 1u)) { failed = true; atomicExch(status, 16); break; }
             have_v = true;
           }
           tcgen05_fence_after();
@@ -258,7 +258,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           __syncwarp();
           if (j + 1 < n_t[x]) {   // the next scores of this tile run under the other tile's softmax
             if (!have_k) {
-              if (!mbar_wait(&bar->k_full[(j + 1) & 1], (uint32_t)((j + 1) >> 1) & 1u)) { failed = true; atomicExch(status, 12); break; }
+              if (!warp_mbar_wait(&bar->k_full[(j + 1) & 1], (uint32_t)((j + 1) >> 1) & 1u)) { failed = true; atomicExch(status, 12); break; }
               have_k = true;
               tcgen05_fence_after();
             }

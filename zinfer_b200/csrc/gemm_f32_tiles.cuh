@@ -53,10 +53,39 @@ struct F32Piece {
   }
 };
 
-// A chunk's pieces (all PIECES of it, or fewer at the end of K) in turn, each read one ahead of its use: a warp or two a
-// scheduler cannot hide the reads otherwise (5 % at 12 x 1024 x 1024, 4 % at 512 x 6144 x 1024).
-template <int TM, int TN, int GAP_A, int GAP_B, int PIECES, int UNROLL>
+// A chunk's pieces (all PIECES of it, or fewer at the end of K) in turn, each read AHEAD pieces before its use: with a warp or
+// two a scheduler nothing else hides a shared-memory read's latency, about ten multiply-adds of a chain.
+template <int TM, int TN, int GAP_A, int GAP_B, int PIECES, int AHEAD>
 __device__ __forceinline__ void f32_chunk(float (&acc)[TM][TN], const float* xs, const float* ws, int pieces) {
+  constexpr int RING = AHEAD + 1;
+  static_assert(PIECES % RING == 0 && PIECES >= RING, "a chunk is a whole number of rings");
+  F32Piece<TM, TN> ring[RING];
+  if (pieces == PIECES) {
+#pragma unroll
+    for (int d = 0; d < AHEAD; ++d) ring[d].template read<GAP_A, GAP_B>(xs, ws, d);
+#pragma unroll 1
+    for (int p = 0; p < PIECES - RING; p += RING) {
+#pragma unroll
+      for (int d = 0; d < RING; ++d) {
+        ring[(d + AHEAD) % RING].template read<GAP_A, GAP_B>(xs, ws, p + d + AHEAD);
+        ring[d].multiply(acc);
+      }
+    }
+    ring[AHEAD].template read<GAP_A, GAP_B>(xs, ws, PIECES - 1);
+#pragma unroll
+    for (int d = 0; d < RING; ++d) ring[d].multiply(acc);
+  } else {
+    for (int p = 0; p < pieces; ++p) {
+      ring[0].template read<GAP_A, GAP_B>(xs, ws, p);
+      ring[0].multiply(acc);
+    }
+  }
+}
+
+// A chunk's pieces (all PIECES of it, or fewer at the end of K) in turn, each read one ahead of its use (512 x 6144 x 1024 195 ->
+// 187 us; with the ring of the kernel for few rows 189, and 512 x 1024 x 3072 125 instead of 120).
+template <int TM, int TN, int GAP_A, int GAP_B, int PIECES, int UNROLL>
+__device__ __forceinline__ void f32_chunk_pairs(float (&acc)[TM][TN], const float* xs, const float* ws, int pieces) {
   F32Piece<TM, TN> even, odd;
   if (pieces == PIECES) {
     even.template read<GAP_A, GAP_B>(xs, ws, 0);
@@ -130,7 +159,7 @@ gemm_f32_tile_kernel(TO* __restrict__ out, const float* __restrict__ x, const fl
     asm volatile("cp.async.commit_group;" ::: "memory");
     const float* xs = f32_smem + (c % STAGES) * T::STAGE + ty * PITCH;
     const float* ws = f32_smem + (c % STAGES) * T::STAGE + (BM + tx) * PITCH;
-    f32_chunk<TM, TN, ROWS_M * PITCH, ROWS_N * PITCH, PIECES, T::UNROLL>(acc, xs, ws, (min(KC, K - c * KC) + 3) / 4);
+    f32_chunk_pairs<TM, TN, ROWS_M * PITCH, ROWS_N * PITCH, PIECES, T::UNROLL>(acc, xs, ws, (min(KC, K - c * KC) + 3) / 4);
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -160,12 +189,12 @@ int launch_f32_tile(void* out, const float* x, const float* w, int M, int N, int
 // Up to 32 rows: the same tiles with a warp of their own for the copies.  One lane per operand row asks for KC columns of
 // it in one untiled bulk copy (both ends on 16-byte boundaries, sizes of whole 16 bytes: K % 4 == 0), so the warps that
 // multiply issue nothing but shared-memory reads and multiply-adds.  Bound by the chain itself: K dependent multiply-adds of
-// four clocks and the reads that feed them (12 x 1024 x 1024: 9.5 us, 4 MB of weights; 18 us with copies by the same warps,
+// four clocks and the reads that feed them (12 x 1024 x 1024: 8.5 us, 4 MB of weights; 9.5 with pieces read one ahead; 18 us with copies by the same warps,
 // whose addresses cost more issue slots than the product).  One tensor copy a chunk in the place of one bulk copy a row,
 // its lines swizzled, was measured too: 11.1 us, for the addresses of the swizzled reads.
-template <int BM_, int BN_, int TM_, int TN_, int KC_, int STAGES_, int UNROLL_>
+template <int BM_, int BN_, int TM_, int TN_, int KC_, int STAGES_, int AHEAD_>
 struct F32Few {
-  static constexpr int BM = BM_, BN = BN_, TM = TM_, TN = TN_, KC = KC_, STAGES = STAGES_, UNROLL = UNROLL_;
+  static constexpr int BM = BM_, BN = BN_, TM = TM_, TN = TN_, KC = KC_, STAGES = STAGES_, AHEAD = AHEAD_;
   static constexpr int WORKERS = (BM / TM) * (BN / TN);
   static constexpr int THREADS = WORKERS + 32;
   static constexpr int PITCH = KC + 4;
@@ -255,7 +284,7 @@ gemm_f32_few_kernel(TO* __restrict__ out, const float* __restrict__ x, const flo
     }
     const float* xs = f32_smem + (size_t)s * T::STAGE + ty * PITCH;
     const float* ws = f32_smem + (size_t)s * T::STAGE + (BM + tx) * PITCH;
-    f32_chunk<TM, TN, ROWS_M * PITCH, ROWS_N * PITCH, KC / 4, T::UNROLL>(acc, xs, ws, min(KC, K - c * KC) / 4);
+    f32_chunk<TM, TN, ROWS_M * PITCH, ROWS_N * PITCH, KC / 4, T::AHEAD>(acc, xs, ws, min(KC, K - c * KC) / 4);
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);
   }

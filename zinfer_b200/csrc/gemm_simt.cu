@@ -224,10 +224,10 @@ namespace {
 // blocks fill the 148 SMs, and the larger a thread's tile the fewer bytes of shared memory it reads per multiply-add
 // (128 bytes a clock and SM feed 4 x 4 outputs a thread at about a third of the multiply-adds' rate, 8 x 8 at half).
 // Measured, us on one B200 (rows x columns x K; the plain kernel -> the tile taken; every output's bits are the same):
-//   1 x 1024 x 1024  106 -> 5.4      12 x 1024 x 1024  106 -> 9.5     12 x 6144 x 1024  126 -> 13.9   12 x 1024 x 3072  311 -> 24.8
-//   30 x 1024 x 1024  12.3           100 x 1024 x 1024  30            512 x 1024 x 1024  101 -> 41    512 x 6144 x 1024  336 -> 187
-// and with the tile next to the line: 12 x 6144 x 1024 in tiles of 8 columns 19.4, 12 x 32768 x 1024 in tiles of 16 68.7
-// against 62.2 of 32; 100 x 1024 x 1024 in 32 x 32 tiles 38; 512 x 1024 x 3072 in 64 x 64 tiles 342 against 120 of 32 x 32,
+//   1 x 1024 x 1024  106 -> 5.4      12 x 1024 x 1024  106 -> 8.5     12 x 6144 x 1024  126 -> 14.2   12 x 1024 x 3072  311 -> 21.7
+//   30 x 1024 x 1024  11.4           100 x 1024 x 1024  26            512 x 1024 x 1024  101 -> 41    512 x 6144 x 1024  336 -> 187
+// and with the tile next to the line: 12 x 6144 x 1024 in tiles of 8 columns 18.3, 12 x 32768 x 1024 in tiles of 16 69.9
+// against 63.1 of 32; 100 x 1024 x 1024 in 32 x 32 tiles 38; 512 x 1024 x 3072 in 64 x 64 tiles 342 against 120 of 32 x 32,
 // 512 x 6144 x 1024 in 32 x 32 tiles 222.
 constexpr int SMS = 148;
 template <typename TO>
@@ -239,19 +239,19 @@ int launch_f32(void* out, const float* x, const float* w, int M, int N, int K, i
     if (!status) return zi_refuse("gemm: no device memory for the status word");
 #define ZI_FEW(...) return launch_f32_few<F32Few<__VA_ARGS__>, TO>(out, x, w, M, N, K, ldx, ldw, ldo, early, status, stream)
     if (M <= 4) {
-      if (N < 32 * SMS) ZI_FEW(4, 8, 1, 1, 256, 4, 8);
-      ZI_FEW(4, 32, 2, 2, 128, 4, 2);
+      if (N < 32 * SMS) ZI_FEW(4, 8, 1, 1, 256, 4, 7);
+      ZI_FEW(4, 32, 2, 1, 128, 4, 7);
     }
     if (M <= 16) {
-      if (N <= 16 * SMS) ZI_FEW(16, 8, 2, 1, 256, 3, 4);
-      if (N <= 80 * SMS) ZI_FEW(16, 16, 2, 2, 128, 4, 4);
-      ZI_FEW(16, 32, 4, 2, 128, 3, 2);
+      if (N <= 16 * SMS) ZI_FEW(16, 8, 2, 1, 256, 3, 3);
+      if (N <= 80 * SMS) ZI_FEW(16, 16, 2, 2, 128, 4, 3);
+      ZI_FEW(16, 32, 2, 2, 128, 3, 3);
     }
     if (M <= 32) {
-      if (N <= 16 * SMS) ZI_FEW(32, 8, 4, 2, 128, 4, 2);
-      ZI_FEW(32, 16, 2, 2, 128, 3, 2);
+      if (N <= 16 * SMS) ZI_FEW(32, 8, 2, 1, 256, 2, 3);
+      ZI_FEW(32, 16, 2, 2, 128, 3, 3);
     }
-    ZI_FEW(32, 16, 4, 4, 128, 3, 2);
+    ZI_FEW(32, 16, 4, 2, 128, 3, 3);
 #undef ZI_FEW
   }
   if (blocks64 >= 5 * SMS) return launch_f32_tile<F32Tile<64, 64, 8, 8, 32, 3, 1>, TO>(out, x, w, M, N, K, ldx, ldw, ldo, early, stream);

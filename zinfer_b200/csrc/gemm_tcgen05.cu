@@ -351,11 +351,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       int a_tile, b_tile, split, kb0, n_kb;
       decode(tile, a_tile, b_tile, split, kb0, n_kb);
       const uint32_t acc = lt & 1u, acc_phase = (lt >> 1) & 1u;
-      if (!mbar_wait(&accum_empty[acc], acc_phase ^ 1u)) { failed = true; atomicExch(status, 4); break; }
+      if (!warp_mbar_wait(&accum_empty[acc], acc_phase ^ 1u)) { failed = true; atomicExch(status, 4); break; }
       tcgen05_fence_after();
       const uint32_t d_tmem = tmem_base + acc * (uint32_t)g.acc_cols;
       for (int i = 0; i < n_kb; ++i) {
-        if (!mbar_wait(&full[s], parity)) { failed = true; atomicExch(status, 2); break; }
+        if (!warp_mbar_wait(&full[s], parity)) { failed = true; atomicExch(status, 2); break; }
         tcgen05_fence_after();
         if (elect_one()) {
           const uint64_t off = (uint64_t)((uint32_t)(s * stage_bytes) >> 4);     // descriptors count 16 bytes
@@ -540,11 +540,11 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       for (int tile = pair; tile < total_tiles && !failed; tile += n_pairs, ++lt) {
         decode(tile, a_tile, b_tile, split, kb0, n_kb);
         const uint32_t acc = lt & 1u, acc_phase = (lt >> 1) & 1u;
-        if (!mbar_wait(&accum_empty[acc], acc_phase ^ 1u)) { failed = true; atomicExch(status, 8); break; }
+        if (!warp_mbar_wait(&accum_empty[acc], acc_phase ^ 1u)) { failed = true; atomicExch(status, 8); break; }
         tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + acc * (uint32_t)PAIR_TILE;
         for (int i = 0; i < n_kb; ++i) {
-          if (!mbar_wait(&full[s], parity)) { failed = true; atomicExch(status, 6); break; }
+          if (!warp_mbar_wait(&full[s], parity)) { failed = true; atomicExch(status, 6); break; }
           tcgen05_fence_after();
           if (elect_one()) {
             const uint64_t off = (uint64_t)((uint32_t)(s * PAIR_STAGE_BYTES) >> 4);
