@@ -581,3 +581,46 @@ def test_recurrence_in_chunks_against_64_bits_and_the_walk(D, V, heads, key_head
     # 2^-22 for the parts' missing products, 2^-24 a rounding: a few of either, as the walk has them
     assert max(got[True]) < 2e-6, got
     assert all(c <= 1.5 * w + 2.0 ** -22 for c, w in zip(got[True], got[False])), got
+
+
+@gpu
+@pytest.mark.parametrize("T,H,splits_a,splits_b", [(1, 4, 1, 0), (8, 2048, 4, 15), (512, 132, 8, 9), (3, 4100, 16, 7), (2, 8192, 0, 3), (5, 1024, 0, 0)])
+def test_norm_of_updates_for_few_rows(T, H, splits_a, splits_b):
+    """Rows held in fours, updates whole or in any number of splits, against 64-bit arithmetic and the form for rows of any
+    width, which rows of the same numbers off the 16-byte boundaries take."""
+    from zinfer_b200 import ops
+
+    gen = torch.Generator(device=DEV).manual_seed(T + H)
+    r = lambda *s: torch.randn(s, generator=gen, device=DEV)
+    form = lambda n: ops.Partials(r(n, T, H)) if n else r(T, H).to(torch.bfloat16)
+    h, w, a, b = r(T, H), 1 + 0.1 * r(H), form(splits_a), form(splits_b)
+    value = lambda u: (u.data.double().sum(0) if isinstance(u, ops.Partials) else u.double())
+    y = 0.7 * value(a) + 1.3 * value(b)
+    want = h.double() + y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5) * w.double()
+    odd = torch.empty(T * H + 1, device=DEV)[1:].view(T, H)          # the stream off the boundary: the general form
+    odd.copy_(h)
+    x = ops.norm_residual(h, ops.Scaled(a, 0.7), w, 1e-5, torch.bfloat16, b=ops.Scaled(b, 1.3))
+    ops.norm_residual(odd, ops.Scaled(a, 0.7), w, 1e-5, torch.bfloat16, b=ops.Scaled(b, 1.3))
+    # sums of at most 31 terms of size about one, a norm over H of them: some tens of roundings of 2^-24
+    assert ((h.double() - want).abs() <= 64 * 2.0 ** -24 * (1 + want.abs())).all()
+    assert ((h - odd).abs() <= 64 * 2.0 ** -24 * (1 + odd.abs())).all()
+    assert torch.equal(x, h.to(torch.bfloat16))
+
+
+@gpu
+@pytest.mark.parametrize("T,N,rank,dim", [(1, 24, 16, 8), (9, 1024, 16, 128), (65, 300, 5, 100), (70, 257, 32, 257), (8, 64, 40, 16)])
+def test_decays_of_a_low_rank_pair(T, N, rank, dim):
+    """One kernel for ranks up to 32 against 64-bit arithmetic, beside the product and the decay's kernel (which a larger
+    rank still takes)."""
+    from zinfer_b200 import ops
+
+    gen = torch.Generator(device=DEV).manual_seed(N)
+    r = lambda *s: torch.randn(s, generator=gen, device=DEV)
+    wide, w = r(T, rank + 11).to(torch.bfloat16), r(N, rank).to(torch.bfloat16)
+    x, bias, a_log = wide[:, 3:3 + rank], r(N), 0.3 * r(N // dim)
+    z = x.double() @ w.double().T + bias.double()
+    want = {None: torch.sigmoid(z) ** (1 / 16.0), 1: torch.exp(-torch.exp(a_log.double()).repeat_interleave(dim) * torch.nn.functional.softplus(z))}
+    for a, exact in want.items():
+        got = ops.low_rank_decay(x, w, bias, a_log if a else None, 16.0, dim)
+        # z of size up to 4 sqrt(rank), its roundings and those of exp, log1p: 2^-18 of the exponent's slope, which is at most |z| e^a
+        assert torch.allclose(got.double(), exact, rtol=2e-5, atol=1e-6)

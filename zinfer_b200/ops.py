@@ -1824,6 +1824,27 @@ def decay_exp_softplus_(z: torch.Tensor, bias: Optional[torch.Tensor], a_log: to
     return z
 
 
+def low_rank_decay(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], a_log: Optional[torch.Tensor], tau: float,
+                   head_dim: int) -> torch.Tensor:
+    """float32 decays [T, N] of ``z = x [T, rank] @ w [N, rank]^T``: with ``a_log`` as :func:`decay_exp_softplus_`, else as
+    :func:`decay_sigmoid_root_` has them.  One kernel for bfloat16 operands of a rank up to 32; otherwise the product and the
+    decay's kernel."""
+    T, rank = x.shape
+    N = w.shape[0]
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and rank <= 32 and x.stride(1) == 1 and w.is_contiguous()
+            and T <= 65535 * 8):
+        z = linear(x, w, out_dtype=torch.float32)
+        return decay_exp_softplus_(z, bias, a_log, head_dim) if a_log is not None else decay_sigmoid_root_(z, bias, tau)
+    _need(w.shape[1] == rank, "low_rank_decay: the two matrices share their rank")
+    for v, n in ((bias, N), (a_log, N // head_dim)):
+        _need(v is None or (v.dtype == torch.float32 and v.numel() == n and v.is_contiguous()), "low_rank_decay: bias and a_log are float32")
+    out = torch.empty((T, N), dtype=torch.float32, device=x.device)
+    with _prof.region("decay (low-rank product)", lambda: _nb(out, w) + T * rank * 2, 2 * T * N * rank):
+        _check(lib().zi_low_rank_decay(_ptr(out), _ptr(x), x.stride(0), _ptr(w), rank, T, N, head_dim, _ptr(bias), _ptr(a_log),
+                                       ctypes.c_float(1.0 / tau), _stream()), "low_rank_decay")
+    return out
+
+
 def unit_norm_(x: torch.Tensor, heads: int, head_dim: int, eps: float, scale: float = 1.0) -> torch.Tensor:
     """In place on float32 rows [T, >= heads * head_dim]: every head ``scale * x / sqrt(sum(x^2) + eps)``."""
     _need(x.dtype == torch.float32 and x.stride(1) == 1 and x.shape[1] >= heads * head_dim, "unit_norm: float32 rows")

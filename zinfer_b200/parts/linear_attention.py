@@ -85,8 +85,7 @@ class GatedLinearAttention(Mixer):
         qk, hv = self.heads * self.dim, self.heads * self.vdim
         proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype)
         q, k, v, g = proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:2 * qk + hv], proj[:, 2 * qk + hv:2 * qk + 2 * hv]
-        z = ops.linear(proj[:, 2 * qk + 2 * hv:], self.w_a2, out_dtype=torch.float32)
-        decay = ops.decay_sigmoid_root_(z, self.a_bias, self.tau)
+        decay = ops.low_rank_decay(proj[:, 2 * qk + 2 * hv:], self.w_a2, self.a_bias, None, self.tau, self.dim)
         o = ops.channel_decay_recurrence(q, k, v, decay, None, self.dim ** -0.5, cache.state, self.heads, self.heads, self.dim, self.vdim, step,
                                          fast=self.ctx.dtype == torch.bfloat16)
         y = ops.head_norm_gate(o, self.norm, self.eps, g, "silu", self.heads, self.vdim, self.ctx.dtype)
@@ -233,12 +232,10 @@ class GatedDeltaRule(Mixer):
         qkv = ops.short_conv(raw, self.conv, tail, step, "silu")                   # float32 [T, C]
         ops.short_conv_carry(raw, self.taps, tail, step)
         q, k, v = qkv[:, :qk], qkv[:, qk:2 * qk], qkv[:, 2 * qk:]
-        ops.unit_norm_(q, self.kv_heads, self.dim, self.UNIT_EPS)
-        ops.unit_norm_(k, self.kv_heads, self.dim, self.UNIT_EPS)
+        ops.unit_norm_(qkv[:, :2 * qk], 2 * self.kv_heads, self.dim, self.UNIT_EPS)      # q's heads, then k's
         beta = ops.sigmoid_rows(proj[:, C:C + H])
         a0 = C + H
-        z = ops.linear(proj[:, a0:a0 + self.decay_rank], self.w_a2, out_dtype=torch.float32)
-        decay = ops.decay_exp_softplus_(z, self.dt_bias, self.a_log, self.dim)
+        decay = ops.low_rank_decay(proj[:, a0:a0 + self.decay_rank], self.w_a2, self.dt_bias, self.a_log, 1.0, self.dim)
         o = ops.channel_decay_recurrence(q, k, v, decay, beta, self.dim ** -0.5, s_view, H, self.kv_heads, self.dim, self.vdim, step,
                                          fast=self.ctx.dtype == torch.bfloat16)
         gate = ops.linear(proj[:, a0 + self.decay_rank:], self.w_g2, out_dtype=self.ctx.dtype)
