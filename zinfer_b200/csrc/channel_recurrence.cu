@@ -23,6 +23,8 @@
 // two remainders is below the sums' rounding), the parts' products are summed apart, and the state is moved on by 32-bit
 // multiply-adds outside of the tensor cores' accumulators.  Against 64 bits outputs and states are as near as the walk's.
 //
+// (A value that is no number reaches the other tokens of its block of 16, also earlier ones: weights of zero meet it there.)
+//
 // A chunk's place in the workspace: request s's chunk i lies at cu_q[s] / 64 + s + i, so that no prefix sum over the
 // requests is needed.  Requests that bring one token are left alone.
 //
