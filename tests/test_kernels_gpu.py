@@ -886,3 +886,17 @@ def test_products_that_the_rule_gives_to_cta_pairs(M, N, K):
             y = o.linear_swiglu(x, o.interleave_gate_up(wg, wu), activation=act)
             torch.testing.assert_close(y.double(), f * u, rtol=1.6e-2, atol=2e-3 * K ** 0.5 * 0.05 + 1e-3)
     assert o.kernel_status() == 0
+
+
+def test_the_first_product_may_lie_in_a_capture():
+    """A process whose first call of the library is a 32-bit product inside a stream capture: the word in which kernels record
+    waits that ran out is made there and then."""
+    import subprocess
+    import sys
+    code = ("import torch\nfrom zinfer_b200 import ops\n"
+            "x, w = torch.ones(3, 64, device='cuda'), torch.ones(5, 64, device='cuda')\n"
+            "ops.lib()\ntorch.cuda.synchronize()\ng = torch.cuda.CUDAGraph()\n"
+            "with torch.cuda.graph(g):\n    y = ops.linear(x, w)\n"
+            "g.replay()\ntorch.cuda.synchronize()\nassert (y == 64).all() and ops.kernel_status() == 0\n")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]

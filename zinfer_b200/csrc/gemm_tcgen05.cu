@@ -680,11 +680,21 @@ int round_up_bn(int n) {
   return 256;
 }
 
+// Made at the first call, which may lie inside a stream capture: this thread may allocate meanwhile, and the word is
+// cleared on a stream of its own.
 int* status_word() {
   static int* word = nullptr;
   static std::once_flag once;
   std::call_once(once, [] {
-    if (cudaMalloc(&word, sizeof(int)) == cudaSuccess) cudaMemset(word, 0, sizeof(int));
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    int* p = nullptr;
+    cudaStream_t own = nullptr;
+    if (cudaMalloc(&p, sizeof(int)) == cudaSuccess && cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) == cudaSuccess &&
+        cudaMemsetAsync(p, 0, sizeof(int), own) == cudaSuccess && cudaStreamSynchronize(own) == cudaSuccess)
+      word = p;
+    if (own) cudaStreamDestroy(own);
+    cudaThreadExchangeStreamCaptureMode(&mode);
   });
   return word;
 }
