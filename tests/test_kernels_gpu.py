@@ -683,6 +683,18 @@ def test_a_wait_that_runs_out_is_reported_not_survived_silently():
         o.selftest_wait_runs_out(code=0)
 
 
+def test_a_warp_answers_a_wait_as_one():
+    """A wait whose limit runs out in half of a warp's lanes fails for all of them, and a producer warp whose elected lane's
+    wait runs out issues nothing more, records the code and still takes all its turns together."""
+    o = ops()
+    assert o.kernel_status() == 0
+    got = o.selftest_waits_of_a_warp(DEV, code=78).tolist()
+    assert got == [0] * 32 + [0, 4]
+    assert o.kernel_status() == 78
+    with pytest.raises(o.KernelError):
+        o.selftest_waits_of_a_warp(DEV, code=0)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T,H,eps", [(3, 72, 1e-6), (7, 4096, 1e-5), (300, 200, 3e-6), (515, 1024, 1e-5), (260, 8192, 1e-6),
                                      (270, 8196, 1e-6), (257, 70, 1e-5)])

@@ -290,7 +290,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     float m_ref = -INFINITY, l = 0.f;
     for (int j = 0; j < nt && !failed; ++j) {
       const int kt = kt0 + j * BK;
-      if (!mbar_wait(s_full, (uint32_t)j & 1u)) { failed = true; atomicExch(status, 18); break; }
+      if (!warp_mbar_wait(s_full, (uint32_t)j & 1u)) { failed = true; atomicExch(status, 18); break; }
       tcgen05_fence_after();
       // Columns c_lo .. c_hi - 1 of this tile are visible to this row; only tiles on the diagonal,
       // at a window's edge or below the first visible key need the test at all (a warp-uniform
@@ -330,7 +330,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         }
         l *= f;
         if (j > 0) {
-          if (!mbar_wait(pv_done, ((uint32_t)j & 1u) ^ 1u)) { failed = true; atomicExch(status, 20); break; }
+          if (!warp_mbar_wait(pv_done, ((uint32_t)j & 1u) ^ 1u)) { failed = true; atomicExch(status, 20); break; }
           tcgen05_fence_after();
 #pragma unroll 1
           for (int c0 = 0; c0 < D; c0 += 32) {
@@ -369,7 +369,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       if (lane == 0) mbar_arrive(p_full);
     }
     if (!failed && nt > 0) {
-      if (!mbar_wait(pv_done, (uint32_t)(nt - 1) & 1u)) { failed = true; atomicExch(status, 21); }
+      if (!warp_mbar_wait(pv_done, (uint32_t)(nt - 1) & 1u)) { failed = true; atomicExch(status, 21); }
       tcgen05_fence_after();
       if (!failed) {
         const float inv = l > 0.f ? 1.0f / l : 0.f;

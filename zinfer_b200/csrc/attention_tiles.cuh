@@ -724,7 +724,7 @@ __device__ __forceinline__ void attn_decode_unit(
     }
     if constexpr (TMA) {
       // the tile's bytes have landed when its barrier's phase completes (bounded wait)
-      if (!mbar_wait(&my_bars[t % STAGES], (uint32_t)(t / STAGES) & 1u)) {
+      if (!warp_mbar_wait(&my_bars[t % STAGES], (uint32_t)(t / STAGES) & 1u)) {
         if (lane == 0 && status) atomicExch(status, 21);
         for (int i = 0; i < 64; ++i) __nanosleep(10000);   // let copies in flight land before the ring is reused
         break;

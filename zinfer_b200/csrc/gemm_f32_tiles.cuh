@@ -254,7 +254,7 @@ gemm_f32_few_kernel(TO* __restrict__ out, const float* __restrict__ x, const flo
       copy_x(c);
     }
     for (int c = ahead; c < chunks; ++c) {
-      if (!mbar_wait(&empty[c % STAGES], ((c / STAGES) & 1) ^ 1)) {
+      if (!mbar_wait(&empty[c % STAGES], ((c / STAGES) & 1) ^ 1)) {     // a lane that gives up leaves; __syncwarp counts those that stay
         failed = true;
         break;
       }
@@ -264,7 +264,7 @@ gemm_f32_few_kernel(TO* __restrict__ out, const float* __restrict__ x, const flo
       copy_x(c);
     }
     if (failed) {                          // copies in flight land before shared memory is given up
-      if (lane == 0) atomicExch(status, 21);
+      atomicExch(status, 21);
       for (int i = 0; i < 64; ++i) __nanosleep(10000);
     }
     return;
@@ -289,7 +289,7 @@ gemm_f32_few_kernel(TO* __restrict__ out, const float* __restrict__ x, const flo
     if (lane == 0) mbar_arrive(&empty[s]);
   }
   if (failed) {
-    if (lane == 0) atomicExch(status, 22);
+    atomicExch(status, 22);
     for (int i = 0; i < 64; ++i) __nanosleep(10000);
     return;
   }

@@ -325,16 +325,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       }
       int s = pre == stages ? 0 : pre;       // the stage of the next k-block, and the parity its last use left
       uint32_t parity = pre == stages ? 0u : 1u;
-      for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
+      for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
         decode(tile, a_tile, b_tile, split, kb0, n_kb);
         for (int i = tile == (int)blockIdx.x ? pre : 0; i < n_kb; ++i) {
-          if (!mbar_wait(&empty[s], parity)) { failed = true; atomicExch(status, 1); break; }
-          if (elect_one()) {
+          elected_turn(&empty[s], parity, failed, status, 1, [&] {
             mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
             issue(1, s, i);
             issue(0, s, i);
-          }
-          __syncwarp();
+          });
           if (++s == stages) {
             s = 0;
             parity ^= 1u;
@@ -381,7 +379,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       int a_tile, b_tile, split, kb0, n_kb;
       decode(tile, a_tile, b_tile, split, kb0, n_kb);
       const uint32_t acc = lt & 1u, acc_phase = (lt >> 1) & 1u;
-      if (!mbar_wait(&accum_full[acc], acc_phase)) { failed = true; atomicExch(status, 3); break; }
+      if (!warp_mbar_wait(&accum_full[acc], acc_phase)) { failed = true; atomicExch(status, 3); break; }
       tcgen05_fence_after();
       int a = a_tile * TILE_A + quarter * 32 + lane;
       TO* out_tile = out;
@@ -514,16 +512,14 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       }
       int s = pre == stages ? 0 : pre;
       uint32_t parity = pre == stages ? 0u : 1u;
-      for (int tile = pair; tile < total_tiles && !failed; tile += n_pairs) {
+      for (int tile = pair; tile < total_tiles; tile += n_pairs) {
         decode(tile, a_tile, b_tile, split, kb0, n_kb);
         for (int i = tile == pair ? pre : 0; i < n_kb; ++i) {
-          if (!mbar_wait(&empty[s], parity)) { failed = true; atomicExch(status, 5); break; }
-          if (elect_one()) {
+          elected_turn(&empty[s], parity, failed, status, 5, [&] {
             if (rank == 0) mbar_expect_tx(&full[s], 2u * (uint32_t)PAIR_STAGE_BYTES);
             issue(1, s, i);
             issue(0, s, i);
-          }
-          __syncwarp();
+          });
           if (++s == stages) {
             s = 0;
             parity ^= 1u;
@@ -570,7 +566,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     for (int tile = pair; tile < total_tiles && !failed; tile += n_pairs, ++lt) {
       decode(tile, a_tile, b_tile, split, kb0, n_kb);
       const uint32_t acc = lt & 1u, acc_phase = (lt >> 1) & 1u;
-      if (!mbar_wait(&accum_full[acc], acc_phase)) { failed = true; atomicExch(status, 7); break; }
+      if (!warp_mbar_wait(&accum_full[acc], acc_phase)) { failed = true; atomicExch(status, 7); break; }
       tcgen05_fence_after();
       const int a = a_tile * PAIR_TILE + (int)rank * TILE_A + quarter * 32 + lane;
       const uint32_t lane_base = tmem_base + acc * (uint32_t)PAIR_TILE + ((uint32_t)(quarter * 32) << 16);
@@ -1186,7 +1182,39 @@ __global__ void wait_that_runs_out_kernel(int* __restrict__ status, int code, ui
     if (!mbar_wait(&bar, 0, tries)) atomicExch(status, code);
   }
 }
+
+// Waits by a whole warp whose limit runs out in half of its lanes only, and turns of a producer warp whose elected lane's
+// wait runs out.  out[0..31]: each lane's answer; out[32], out[33]: turns issued of four with a limit of 0 and of `tries`.
+__global__ void waits_of_a_warp_kernel(int* __restrict__ status, int code, uint32_t tries, int* __restrict__ out) {
+  __shared__ __align__(8) uint64_t bar;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_arrive(&bar);
+  }
+  __syncthreads();
+  const bool ok = warp_mbar_wait(&bar, 0, lane < 16 ? 0u : tries);
+  out[lane] = ok ? 1 : 0;
+  if (!ok) atomicExch(status, code);
+  for (int round = 0; round < 2; ++round) {
+    bool failed = false;
+    int issued = 0;
+    for (int i = 0; i < 4; ++i) elected_turn(&bar, 0, failed, status, code, [&] { ++issued; }, round ? tries : 0u);
+    issued = __reduce_add_sync(0xffffffffu, issued);
+    if (lane == 0) out[32 + round] = issued;
+  }
+}
 }  // namespace
+
+extern "C" int zi_selftest_waits_of_a_warp(int code, int tries, int* out, cudaStream_t stream) {
+  if (code == 0 || tries <= 0 || tries > (1 << 20) || !out)
+    return zi_refuse("selftest_waits_of_a_warp: code must be non-zero, tries in 1..2^20, and 34 words for the answers");
+  int* status = status_word();
+  if (!status) return zi_refuse("selftest_waits_of_a_warp: cannot allocate the status word");
+  waits_of_a_warp_kernel<<<1, 32, 0, stream>>>(status, code, (uint32_t)tries, out);
+  return zi_check_launch("selftest_waits_of_a_warp");
+}
 
 extern "C" int zi_selftest_wait_runs_out(int code, int tries, cudaStream_t stream) {
   if (code == 0 || tries <= 0 || tries > (1 << 20))

@@ -46,10 +46,26 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
   return p != 0;
 }
-// A wait by a whole warp whose answer the compiler knows to be the same in all lanes, so that a loop which ends with it keeps
-// its counters in the warp's registers (a k-block of four small MMAs 0.26 -> 0.225 us; without effect where the tensor
-// cores set the pace, and slower where only copies are issued).
-__device__ __forceinline__ bool warp_mbar_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+// A wait by a whole warp with one answer for all its lanes.  Each lane counts its own tries, so a wait that runs out may do so
+// in some lanes while the barrier flips for the others; a warp that parted there would meet its next warp-wide instruction
+// (elect.sync, a tensor-memory load, __syncwarp) incomplete.  A loop which ends with this answer also keeps its counters in
+// the warp's registers (a k-block of four small MMAs 0.26 -> 0.225 us).
+__device__ __forceinline__ bool warp_mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = WAIT_LIMIT) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit));
+}
+// A producer warp's turn at a stage: its lanes wait, each by its own tries, and the elected one issues.  A lane whose wait runs
+// out records `code` and from then on neither waits nor issues, but takes every further turn with the others: no loop may end
+// on `failed`.  (A vote on every wait, as above, costs where only copies are issued: 0.5 to 1 % of a product of few tokens.)
+template <typename F>
+__device__ __forceinline__ void elected_turn(uint64_t* bar, uint32_t parity, bool& failed, int* status, int code, F issue,
+                                             uint32_t limit = WAIT_LIMIT) {
+  if (!failed && !mbar_wait(bar, parity, limit)) {
+    failed = true;
+    atomicExch(status, code);
+  }
+  if (elect_one() && !failed) issue();
+  __syncwarp();
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"

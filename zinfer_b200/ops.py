@@ -65,6 +65,14 @@ def selftest_wait_runs_out(code: int = 77, tries: int = 4096) -> None:
     _check(lib().zi_selftest_wait_runs_out(code, tries, _stream()), "selftest_wait_runs_out")
 
 
+def selftest_waits_of_a_warp(device, code: int = 77, tries: int = 4096) -> torch.Tensor:
+    """Waits on a barrier that has been arrived at, with a limit of 0 for half of a warp's lanes: int32 [34], each lane's answer
+    and how many of four turns the warp's elected lane issued with a limit of 0 and of ``tries``.  Leaves ``code`` behind."""
+    out = torch.full((34,), -1, dtype=torch.int32, device=device)
+    _check(lib().zi_selftest_waits_of_a_warp(code, tries, _ptr(out), _stream()), "selftest_waits_of_a_warp")
+    return out
+
+
 def gemm_pair_kernel(on: bool) -> bool:
     """Switches the matrix product's kernel for CTA pairs (tcgen05 ``cta_group::2``: two SMs on one
     tile of 256 tokens x 256 weight rows, each loading half of the weight rows) on for all products of
