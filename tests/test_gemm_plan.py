@@ -45,6 +45,25 @@ def test_many_tokens_are_left_whole_and_a_few_hundred_are_split_when_it_pays(pla
     assert plan(512, 24576, 4096)["splits"] == 1
 
 
+def test_without_room_for_a_cluster_products_stay_with_the_single_cta_kernel():
+    """CTA pairs are planned for the clusters that the GPU holds: none of them, no pairs, and the plan is the single kernel's."""
+    if shutil.which("nvcc") is None:
+        pytest.skip("no nvcc to build the kernel library with")
+    from zinfer_b200 import ops
+
+    def f(M, N, K, pairs):
+        out = (ctypes.c_int * 4)()
+        ops.lib().zi_gemm_tcgen05_plan_for(M, N, K, 148, pairs, out)
+        return tuple(out)
+
+    for M, N, K in [(300, 4096, 12288), (536, 4096, 12288), (2048, 24576, 4096)]:
+        assert f(M, N, K, 74)[3] == 1
+        swap, BN, splits, pair = f(M, N, K, 0)
+        assert pair == 0 and swap == 0 and BN in (128, 256) and splits >= 1
+    assert f(2048, 24576, 4096, 20)[3] == 0        # 768 tiles in 39 rounds of 20 against 6 of 148 with twice the tiles each
+    assert f(128, 24576, 4096, 74)[3] == 0
+
+
 def test_splits_never_leave_a_split_without_k_blocks(plan):
     for M in (1, 8, 64, 65, 128, 300):
         for N, K in [(128, 64), (256, 512), (1000, 264), (4096, 4096), (5120, 17408), (151936, 4096)]:

@@ -710,6 +710,47 @@ extern "C" int zi_gemm_tcgen05_supported(const void* x, const void* w, int K, in
          encode_fn() != nullptr;
 }
 
+namespace {
+constexpr int PAIR_STAGES = 6;
+size_t pair_smem(int stages) { return 1024 + (size_t)stages * PAIR_STAGE_BYTES + (2 * stages + 4) * sizeof(uint64_t) + 16; }
+
+// Clusters of two CTAs of the kernel for pairs that the current device holds at once (74 on 148 SMs), asked once per device with
+// the most shared memory a launch takes; all instances have the same threads and one CTA an SM.  0 where none fits, or
+// the device cannot say: the product then stays with the single-CTA kernel.  Without a device (plans alone): half the SMs.
+int resident_pairs(int sm_count) {
+  static std::mutex mu;
+  static int resident[64];      // 0 = not asked yet, else the answer + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return (sm_count > 0 ? sm_count : 148) / 2;
+  }
+  if (dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  if (resident[dev] == 0) {
+    auto kern = gemm_tcgen05_pair_kernel<float, EPI_PLAIN>;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(2 * 148);
+    cfg.blockDim = dim3(PAIR_THREADS);
+    cfg.dynamicSmemBytes = pair_smem(PAIR_STAGES);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    resident[dev] = n + 1;
+  }
+  return resident[dev] - 1;
+}
+}  // namespace
+
 // The plan of the single-CTA kernel, {swap, BN, splits}.
 static void plan_single(int M, int N, int K, int sm_count, int* plan) {
   const int k_blocks = (K + BLOCK_K - 1) / BLOCK_K;
@@ -779,13 +820,14 @@ int g_pair_mode = -1;
 // (or 128 x 128) tile takes 0.37 (0.31) us, of a pair's 256 x 256 tile 0.335 us (measured on full rounds of real weights; with
 // operands from L2 0.32, 0.31 and 0.29).  Splitting K writes the sums as floats and reads them back, about 6 TB/s in L2,
 // and 3 us more; it has to promise 8 us, for the model is no better than that.  Measured, us (single -> pair): 2048 x 24576 x
-// 4096 282 -> 265, 2048 x 4096 x 12288 156 -> 144, 1024 x 4096 x 12288 80 -> 74, 512 x 24576 x 4096 89 -> 80.
-bool plan_pair(int M, int N, int K, int sm_count, int* plan) {
+// 4096 282 -> 265, 2048 x 4096 x 12288 156 -> 144, 1024 x 4096 x 12288 80 -> 74, 512 x 24576 x 4096 89 -> 80.  `slots`: pairs
+// resident at once (resident_pairs).
+bool plan_pair(int M, int N, int K, int sm_count, int slots, int* plan) {
   if (g_pair_mode < 0) {
     const char* e = getenv("ZINFER_B200_GEMM_PAIR");
     g_pair_mode = e && e[0] == '1' ? PAIR_ALWAYS : (e && e[0] == '0' ? PAIR_NEVER : PAIR_AUTO);
   }
-  if (g_pair_mode == PAIR_NEVER || plan[0] || N < PAIR_TILE) return false;
+  if (g_pair_mode == PAIR_NEVER || plan[0] || N < PAIR_TILE || slots <= 0) return false;
   if (g_pair_mode == PAIR_ALWAYS) {
     // as far as it wastes little: 300 tokens would fill 512 rows of pair tiles but 384 of single tiles
     const int pair_rows = (M + PAIR_TILE - 1) / PAIR_TILE * PAIR_TILE, single_rows = (M + TILE_A - 1) / TILE_A * TILE_A;
@@ -800,11 +842,11 @@ bool plan_pair(int M, int N, int K, int sm_count, int* plan) {
   const long long singles = (long long)((M + TILE_A - 1) / TILE_A) * ((N + plan[1] - 1) / plan[1]);
   const long long pairs = (long long)((M + PAIR_TILE - 1) / PAIR_TILE) * ((N + PAIR_TILE - 1) / PAIR_TILE);
   const double single = time(singles, sms, plan[2], plan[1] >= 256 ? 0.37 : 0.31);
-  const double whole = time(pairs, sms / 2, 1, 0.335);
+  const double whole = time(pairs, slots, 1, 0.335);
   double best = whole;
   int splits = 1;
   for (int s = 2; s <= 8 && k_blocks / s >= 8; ++s) {
-    const double t = time(pairs, sms / 2, s, 0.335);
+    const double t = time(pairs, slots, s, 0.335);
     if (t < best && t < whole - 8.0) {
       best = t;
       splits = s;
@@ -825,16 +867,20 @@ bool plan_pair(int M, int N, int K, int sm_count, int* plan) {
 // `plan` receives {swap, BN, splits}.
 extern "C" long long zi_gemm_tcgen05_plan(int M, int N, int K, int sm_count, int* plan) {
   plan_single(M, N, K, sm_count, plan);
-  plan_pair(M, N, K, sm_count, plan);
+  plan_pair(M, N, K, sm_count, resident_pairs(sm_count), plan);
   return plan[2] > 1 ? (long long)plan[2] * M * N * (long long)sizeof(float) : 0;
+}
+// The same for a GPU that holds `pair_slots` pairs of CTAs at once; `plan` receives {swap, BN, splits, on pairs}.
+extern "C" void zi_gemm_tcgen05_plan_for(int M, int N, int K, int sm_count, int pair_slots, int* plan) {
+  plan_single(M, N, K, sm_count, plan);
+  plan[3] = plan_pair(M, N, K, sm_count, pair_slots, plan);
 }
 
 namespace {
 // Rows of the B side's copy box.
 int b_box_rows(const int* plan, bool pair) { return pair ? PAIR_TILE / 2 : plan[1]; }
 
-// Launch of the pair kernel: clusters of two CTAs, as many as are resident at once (74 on 148 SMs).
-// Returns -3 when no cluster fits (the caller then has no maps for the single kernel: an error).
+// Launch of the pair kernel: clusters of two CTAs, as many as are resident at once.
 template <typename TO, int EPI>
 int launch_pair(void* out, const CUtensorMap& map_a, const CUtensorMap& map_b, GemmArgs g, float* partial, int M, int N,
                 int* status, const char* what, cudaStream_t stream) {
@@ -842,9 +888,9 @@ int launch_pair(void* out, const CUtensorMap& map_a, const CUtensorMap& map_b, G
   g.b_tiles = (N + PAIR_TILE - 1) / PAIR_TILE;
   g.BN = PAIR_TILE;
   g.acc_cols = PAIR_TILE;
-  g.stages = 6;
+  g.stages = PAIR_STAGES;
   if (g.stages > g.k_blocks_per_split) g.stages = g.k_blocks_per_split < 2 ? 2 : g.k_blocks_per_split;
-  const size_t smem = 1024 + (size_t)g.stages * PAIR_STAGE_BYTES + (2 * g.stages + 4) * sizeof(uint64_t) + 16;
+  const size_t smem = pair_smem(g.stages);
   auto kern = gemm_tcgen05_pair_kernel<TO, EPI>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return zi_refuse("%s: cannot get %zu bytes of shared memory", what, smem);
@@ -860,27 +906,7 @@ int launch_pair(void* out, const CUtensorMap& map_a, const CUtensorMap& map_b, G
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  // clusters resident at once: asked once per device, kernel and number of stages (no allocation here:
-  // this path also serves callers that must not allocate)
-  static std::mutex mu;
-  static int resident[64][8];   // of this instance; 0 = not asked yet, else the answer + 1
-  int clusters = 0, dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return zi_refuse("%s: no current device", what);
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    int& slot = resident[dev][g.stages];
-    if (slot == 0) {
-      cfg.gridDim = dim3(2 * 148);
-      cfg.numAttrs = 1;
-      int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-      }
-      slot = n + 1;
-    }
-    clusters = slot - 1;
-  }
+  int clusters = resident_pairs(0);
   if (clusters <= 0) return zi_refuse("%s: no cluster of two CTAs fits on this GPU", what);
   const int total_tiles = g.a_tiles * g.b_tiles * g.splits;
   if (clusters > total_tiles) clusters = total_tiles;
@@ -1024,7 +1050,7 @@ extern "C" int zi_gemm_tcgen05(void* out, int out_dtype, const void* x, const vo
   plan_single(M, N, K, sm_count, plan);
   // (the kernel for pairs asks for its first weight tiles before the wait for the kernels before it; where `w` is written by one
   // of them the sums' splits are still the plan's)
-  const bool pair = plan_pair(M, N, K, sm_count, plan) && !((defer_reduce >> 1) & 1);
+  const bool pair = plan_pair(M, N, K, sm_count, resident_pairs(sm_count), plan) && !((defer_reduce >> 1) & 1);
   const long long need = plan[2] > 1 ? (long long)plan[2] * M * N * (long long)sizeof(float) : 0;
   if (need > workspace_bytes) return zi_refuse("gemm_tcgen05: split-K needs %lld workspace bytes, got %lld", need, workspace_bytes);
   const int swap = plan[0];
@@ -1103,7 +1129,7 @@ extern "C" int zi_gemm_tcgen05_gated(void* out, int out_dtype, const void* x, co
     return zi_refuse("gemm_swiglu: operands must be 16-byte aligned bfloat16 with row pitches in multiples of 8");
   int plan[3];
   plan_single(M, N2, K, sm_count, plan);
-  const bool pair = plan_pair(M, N2, K, sm_count, plan);
+  const bool pair = plan_pair(M, N2, K, sm_count, resident_pairs(sm_count), plan);
   if (plan[2] > 1) return -2;
   const int swap = plan[0];
   // Few tokens: the separate SwiGLU kernel is the better schedule.  While it runs, the CTAs of
