@@ -584,6 +584,49 @@ def test_recurrence_in_chunks_against_64_bits_and_the_walk(D, V, heads, key_head
 
 
 @gpu
+@pytest.mark.parametrize("delta", [False, True])
+@pytest.mark.parametrize("what", ["q", "k", "v", "decay", "beta", "state"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+def test_values_that_are_no_numbers_reach_in_chunks_what_they_reach_token_by_token(delta, what, bad):
+    """One value that is no number or infinite in the middle of a block of 16 tokens: earlier tokens, other heads and
+    other requests keep their results, later ones and the state get numbers, infinities and NaNs where the walk has them."""
+    from zinfer_b200 import ops
+
+    if what == "beta" and not delta:
+        pytest.skip("no such operand")
+    D, V, H = 32, 24, 2
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    q_lens, slots = [200, 90, 1], [1, 0, 2]
+    T, hit, head = sum(q_lens), 71, 1
+    r = lambda *s: torch.randn(s, generator=gen, device=DEV)
+    args = {"q": r(T, H * D), "k": r(T, H * D) / D ** 0.5, "v": r(T, H * V), "decay": torch.sigmoid(2 + r(T, H * D)),
+            "beta": torch.sigmoid(r(T, H)) if delta else None, "state": 0.3 * r(4, H, D, V)}
+    clean = {n: None if a is None else a.clone() for n, a in args.items()}
+    if what == "state":
+        args["state"][1, head, 3, 5] = bad
+    elif what == "beta":
+        args["beta"][hit, head] = bad
+    else:
+        args[what][hit, head * (V if what == "v" else D) + 3] = bad
+    step = _step(q_lens, slots)
+    step.max_q_len, step.n_dec = max(q_lens), 1
+
+    def run(a, fast):
+        state = a["state"].clone()
+        o = ops.channel_decay_recurrence(a["q"], a["k"], a["v"], a["decay"], a["beta"], 0.5, state, H, H, D, V, step, fast=fast)
+        return o.view(T, H, V), state
+
+    (o, s), (wo, ws), (co, cs) = run(args, True), run(args, False), run(clean, True)
+    for got, want in ((o, wo), (s, ws)):
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
+        ok = want.isfinite() & (want.abs() < 1e30)
+        torch.testing.assert_close(got[ok], want[ok], rtol=1e-4, atol=1e-4)
+    first = 0 if what == "state" else hit
+    assert torch.equal(o[200:], co[200:]) and torch.equal(o[:, 1 - head], co[:, 1 - head]) and torch.equal(s[[0, 2, 3]], cs[[0, 2, 3]])
+    assert o[:first].isfinite().all() and not torch.equal(o[first:200, head], co[first:200, head])
+
+
+@gpu
 @pytest.mark.parametrize("T,H,splits_a,splits_b", [(1, 4, 1, 0), (8, 2048, 4, 15), (512, 132, 8, 9), (3, 4100, 16, 7), (2, 8192, 0, 3), (5, 1024, 0, 0)])
 def test_norm_of_updates_for_few_rows(T, H, splits_a, splits_b):
     """Rows held in fours, updates whole or in any number of splits, against 64-bit arithmetic and the form for rows of any

@@ -23,7 +23,9 @@
 // two remainders is below the sums' rounding), the parts' products are summed apart, and the state is moved on by 32-bit
 // multiply-adds outside of the tensor cores' accumulators.  Against 64 bits outputs and states are as near as the walk's.
 //
-// (A value that is no number reaches the other tokens of its block of 16, also earlier ones: weights of zero meet it there.)
+// A value that is infinite or no number would reach earlier tokens too (zero weights meet it in P U) and infinities would
+// not survive the split into parts.  So a block of the walk whose outputs or state come out so takes its request, head and
+// value channels again token by token from the state it began with (walk_tokens), as the recurrence is written.
 //
 // A chunk's place in the workspace: request s's chunk i lies at cu_q[s] / 64 + s + i, so that no prefix sum over the
 // requests is needed.  Requests that bring one token are left alone.
@@ -46,6 +48,7 @@ struct ChannelJob {
   const float* decay;  // [T][H * D]
   const float* beta;   // [T][H] or null
   int ldq, ldk, ldv, ldg, ldb;
+  int qk_dtype;
   float q_scale;
   float* state;
   long long slot_stride;
@@ -377,9 +380,63 @@ size_t channel_walk_smem(int D, bool delta) {
   return (rows * (delta ? 2 : 1) + 2 * keys + 2 * p + 2 * D + (size_t)2 * (D + RK) * SP) * sizeof(float);
 }
 
+// The recurrence token by token with plain 32-bit multiply-adds, in the walk's own form (linear_attention.cu: read out the decayed
+// state, then what the token adds), for value channels v0 .. v0 + RV - 1 of a head, by the whole block: a thread holds the key
+// channels tid / RV + 32 r of one value channel.  For portions that hold values which are no numbers; `red` is
+// [3][WK_THREADS / 32][RV] of shared memory.
+template <typename TV, bool DELTA>
+__device__ __noinline__ void walk_tokens(const ChannelJob& j, float* state, float* red, int tok0, int qlen, int h, int v0) {
+  constexpr int GROUPS = WK_THREADS / RV, ROWS = 128 / GROUPS, WARPS = WK_THREADS / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c = tid % RV, col = v0 + c, i0 = tid / RV, g = h / (j.H / j.G);
+  const bool on = col < j.V;
+  auto key = [&](const void* p, int ld, int t, int i) {
+    const size_t at = (size_t)(tok0 + t) * ld + (size_t)g * j.D + i;
+    return j.qk_dtype == ZI_F32 ? static_cast<const float*>(p)[at] : to_f32(static_cast<const __nv_bfloat16*>(p)[at]);
+  };
+  float st[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) st[r] = on && i0 + r * GROUPS < j.D ? state[(size_t)(i0 + r * GROUPS) * j.V + col] : 0.f;
+  for (int t = 0; t < qlen; ++t) {
+    float kt[ROWS], sum[3] = {0.f, 0.f, 0.f};         // (g S)^T k, (g S)^T q, k . q
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const int i = i0 + r * GROUPS;
+      kt[r] = 0.f;
+      if (i >= j.D) continue;
+      const float qt = key(j.q, j.ldq, t, i) * j.q_scale;
+      kt[r] = key(j.k, j.ldk, t, i);
+      st[r] *= j.decay[(size_t)(tok0 + t) * j.ldg + (size_t)h * j.D + i];
+      if (DELTA) sum[0] = fmaf(st[r], kt[r], sum[0]);
+      sum[1] = fmaf(st[r], qt, sum[1]);
+      sum[2] = fmaf(kt[r], qt, sum[2]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+      sum[n] += __shfl_xor_sync(0xffffffffu, sum[n], RV);
+      if (lane < RV) red[(n * WARPS + warp) * RV + c] = sum[n];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+      sum[n] = 0.f;
+      for (int w = 0; w < WARPS; ++w) sum[n] += red[(n * WARPS + w) * RV + c];
+    }
+    float u = on ? to_f32(static_cast<const TV*>(j.v)[(size_t)(tok0 + t) * j.ldv + (size_t)h * j.V + col]) : 0.f;
+    if (DELTA) u -= sum[0];
+    if (j.beta) u *= j.beta[(size_t)(tok0 + t) * j.ldb + h];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) st[r] = fmaf(kt[r], u, st[r]);
+    if (on && i0 == 0) j.out[(size_t)(tok0 + t) * j.ldo + (size_t)h * j.V + col] = fmaf(u, sum[2], sum[1]);
+  }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+    if (on && i0 + r * GROUPS < j.D) state[(size_t)(i0 + r * GROUPS) * j.V + col] = st[r];
+}
+
 template <typename TV, bool DELTA>
 __global__ void __launch_bounds__(WK_THREADS)
-channel_walk_kernel(const ChannelJob j) {
+channel_walk_kernel(const __grid_constant__ ChannelJob j) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) float wk[];
   const int D = j.D, QP = D + 4, KP = D + 8, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wr = warp & 3, wc = ((warp >> 2) & 1) * 8;
@@ -477,6 +534,7 @@ channel_walk_kernel(const ChannelJob j) {
   const int frag = fk * SP + wc + fr;                // this lane's place in 8 rows of S or U
 
   TwoSums sum;
+  bool finite = true;                                // the outputs, and at the end the state: neither forgets a value that is no number
   for (int i = 0; i < chunks; ++i) {
     const int n = min(RK, qlen - i * RK), first = tok0 + i * RK, buf = i & 1;
     // what becomes U: asked for now, needed after the product with the state
@@ -518,7 +576,11 @@ channel_walk_kernel(const ChannelJob j) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int t = wr * 16 + fr + (e >> 1) * 8, col = v0 + fc + (e & 1);
-        if (t < n && col < j.V) j.out[(size_t)(first + t) * j.ldo + (size_t)h * j.V + col] = sum.sum(e);
+        const float o = sum.sum(e);
+        if (t < n && col < j.V) {
+          j.out[(size_t)(first + t) * j.ldo + (size_t)h * j.V + col] = o;
+          finite &= isfinite(o);
+        }
       }
     } else {
       const float* Kb = K + buf * RK * KP + fk * KP + fr;
@@ -535,6 +597,11 @@ channel_walk_kernel(const ChannelJob j) {
       }
       if (i + 1 < chunks) share_state();
     }
+  }
+  each([&](float& x, float*) { finite &= isfinite(x); });
+  if (__syncthreads_or(!finite)) {
+    walk_tokens<TV, DELTA>(j, state, wk, tok0, qlen, h, v0);
+    return;
   }
   each([](float& x, float* at) { *at = x; });
 }
@@ -576,7 +643,7 @@ extern "C" int zi_channel_recurrence(float* out, int ldo, const void* q, int ldq
   const ChannelPlan p = channel_plan(places, H, D, V, delta);
   ChannelJob j = {};
   j.q = q; j.k = k; j.v = v; j.decay = decay; j.beta = beta;
-  j.ldq = ldq; j.ldk = ldk; j.ldv = ldv; j.ldg = ldg; j.ldb = ldb; j.q_scale = q_scale;
+  j.ldq = ldq; j.ldk = ldk; j.ldv = ldv; j.ldg = ldg; j.ldb = ldb; j.qk_dtype = qk_dtype; j.q_scale = q_scale;
   j.state = state; j.slot_stride = slot_stride; j.H = H; j.G = G; j.D = D; j.V = V;
   j.cu_q = cu_q; j.state_slots = state_slots; j.n_seqs = n_seqs; j.out = out; j.ldo = ldo;
   float* at = workspace;
