@@ -64,6 +64,21 @@ def test_without_room_for_a_cluster_products_stay_with_the_single_cta_kernel():
     assert f(128, 24576, 4096, 74)[3] == 0
 
 
+def test_a_product_with_a_fresh_weight_keeps_the_single_kernels_plan():
+    """Where ``w`` is written earlier in the step the single-CTA kernel runs, by its own tile and splits and not by those of
+    the pairs that the rule would have chosen."""
+    if shutil.which("nvcc") is None:
+        pytest.skip("no nvcc to build the kernel library with")
+    from zinfer_b200 import ops
+
+    for M, N, K in [(130, 4096, 4096), (300, 1024, 12288), (536, 4096, 12288), (257, 2050, 8200), (1024, 1280, 4160), (2048, 512, 2048)]:
+        single, fresh = (ctypes.c_int * 4)(), (ctypes.c_int * 3)()
+        ops.lib().zi_gemm_tcgen05_plan_for(M, N, K, 148, 0, single)
+        need = ops.lib().zi_gemm_tcgen05_plan_fresh(M, N, K, 148, fresh)
+        assert tuple(fresh) == tuple(single)[:3] and single[3] == 0
+        assert need == (4 * fresh[2] * M * N if fresh[2] > 1 else 0)
+
+
 def test_splits_never_leave_a_split_without_k_blocks(plan):
     for M in (1, 8, 64, 65, 128, 300):
         for N, K in [(128, 64), (256, 512), (1000, 264), (4096, 4096), (5120, 17408), (151936, 4096)]:

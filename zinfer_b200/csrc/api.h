@@ -92,6 +92,7 @@ int zi_rglru_decode(void* out, int ldo, const void* yx, int ld, int dtype, const
 
 int zi_gemm_tcgen05_supported(const void* x, const void* w, int K, int ldx, int ldw);
 long long zi_gemm_tcgen05_plan(int M, int N, int K, int sm_count, int* plan);
+long long zi_gemm_tcgen05_plan_fresh(int M, int N, int K, int sm_count, int* plan);
 void zi_gemm_tcgen05_plan_for(int M, int N, int K, int sm_count, int pair_slots, int* plan);
 int zi_gemm_tcgen05(void* out, int out_dtype, const void* x, const void* w, int M, int N, int K, int ldx, int ldw,
                     int ldo, float* workspace, long long workspace_bytes, int sm_count, int defer_reduce,

@@ -870,7 +870,12 @@ extern "C" long long zi_gemm_tcgen05_plan(int M, int N, int K, int sm_count, int
   plan_pair(M, N, K, sm_count, resident_pairs(sm_count), plan);
   return plan[2] > 1 ? (long long)plan[2] * M * N * (long long)sizeof(float) : 0;
 }
-// The same for a GPU that holds `pair_slots` pairs of CTAs at once; `plan` receives {swap, BN, splits, on pairs}.
+// The same for a product whose `w` is written by a kernel of the same step, which takes the single-CTA kernel by its own plan.
+extern "C" long long zi_gemm_tcgen05_plan_fresh(int M, int N, int K, int sm_count, int* plan) {
+  plan_single(M, N, K, sm_count, plan);
+  return plan[2] > 1 ? (long long)plan[2] * M * N * (long long)sizeof(float) : 0;
+}
+// The plan for a GPU that holds `pair_slots` pairs of CTAs at once; `plan` receives {swap, BN, splits, on pairs}.
 extern "C" void zi_gemm_tcgen05_plan_for(int M, int N, int K, int sm_count, int pair_slots, int* plan) {
   plan_single(M, N, K, sm_count, plan);
   plan[3] = plan_pair(M, N, K, sm_count, pair_slots, plan);
@@ -1048,9 +1053,8 @@ extern "C" int zi_gemm_tcgen05(void* out, int out_dtype, const void* x, const vo
     return zi_refuse("gemm_tcgen05: operands must be 16-byte aligned bfloat16 with row pitches in multiples of 8");
   int plan[3];
   plan_single(M, N, K, sm_count, plan);
-  // (the kernel for pairs asks for its first weight tiles before the wait for the kernels before it; where `w` is written by one
-  // of them the sums' splits are still the plan's)
-  const bool pair = plan_pair(M, N, K, sm_count, resident_pairs(sm_count), plan) && !((defer_reduce >> 1) & 1);
+  // (the kernel for pairs asks for its first weight tiles before the wait for the kernels before it: not where one of them writes `w`)
+  const bool pair = !((defer_reduce >> 1) & 1) && plan_pair(M, N, K, sm_count, resident_pairs(sm_count), plan);
   const long long need = plan[2] > 1 ? (long long)plan[2] * M * N * (long long)sizeof(float) : 0;
   if (need > workspace_bytes) return zi_refuse("gemm_tcgen05: split-K needs %lld workspace bytes, got %lld", need, workspace_bytes);
   const int swap = plan[0];

@@ -36,6 +36,7 @@ def lib() -> ctypes.CDLL:
             raise KernelError(f"cannot load the kernel library {path}: {e}") from None
         _LIB.zi_last_error.restype = ctypes.c_char_p
         _LIB.zi_gemm_tcgen05_plan.restype = ctypes.c_longlong
+        _LIB.zi_gemm_tcgen05_plan_fresh.restype = ctypes.c_longlong
         _LIB.zi_attention_decode_workspace_floats.restype = ctypes.c_longlong
         _LIB.zi_linear_recurrence_tiles_floats.restype = ctypes.c_longlong
         _LIB.zi_channel_recurrence_workspace_floats.restype = ctypes.c_longlong
@@ -785,7 +786,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
             and lib().zi_gemm_tcgen05_supported(_ptr(x), _ptr(weight), K, x.stride(0), weight.stride(0))):
         plan = (ctypes.c_int * 3)()
         sms = _sm_count(x.device)
-        need = lib().zi_gemm_tcgen05_plan(M, N, K, sms, plan)
+        need = (lib().zi_gemm_tcgen05_plan_fresh if fresh_weight else lib().zi_gemm_tcgen05_plan)(M, N, K, sms, plan)
         ws = torch.empty((need // 4,), dtype=torch.float32, device=x.device) if need else None
         defer = allow_partials and need > 0 and out is None
         if out is None and not defer:
