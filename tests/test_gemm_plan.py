@@ -79,6 +79,27 @@ def test_a_product_with_a_fresh_weight_keeps_the_single_kernels_plan():
         assert need == (4 * fresh[2] * M * N if fresh[2] > 1 else 0)
 
 
+@pytest.mark.parametrize("env,first", [(None, None), ("0", False), ("1", True)])
+def test_the_switch_of_cta_pairs_gives_back_what_it_found(env, first):
+    """Never, always, by the rule: the setting before, the environment's at first, comes back and is what the plans follow."""
+    import os
+    import subprocess
+    import sys
+    if shutil.which("nvcc") is None:
+        pytest.skip("no nvcc to build the kernel library with")
+    code = ("import ctypes\nfrom zinfer_b200 import ops\n"
+            "def pairs(M, N, K):\n    p = (ctypes.c_int * 4)()\n    ops.lib().zi_gemm_tcgen05_plan_for(M, N, K, 148, 74, p)\n    return bool(p[3])\n"
+            "shapes = [(2048, 24576, 4096), (384, 12288, 4096), (512, 256, 256)]\n"
+            "found = [pairs(*s) for s in shapes]\n"
+            f"assert ops.gemm_pair_kernel(False) is {first}\nassert not any(pairs(*s) for s in shapes)\n"
+            "assert ops.gemm_pair_kernel(True) is False\nassert all(pairs(*s) for s in shapes[::2])\n"
+            f"assert ops.gemm_pair_kernel({first}) is True\nassert [pairs(*s) for s in shapes] == found\n"
+            "assert ops.gemm_pair_kernel(None) is " + str(first) + "\nassert pairs(*shapes[0])\nassert ops.gemm_pair_kernel(False) is None\n")
+    env = {**{k: v for k, v in os.environ.items() if k != "ZINFER_B200_GEMM_PAIR"}, **({} if env is None else {"ZINFER_B200_GEMM_PAIR": env})}
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, env=env)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_splits_never_leave_a_split_without_k_blocks(plan):
     for M in (1, 8, 64, 65, 128, 300):
         for N, K in [(128, 64), (256, 512), (1000, 264), (4096, 4096), (5120, 17408), (151936, 4096)]:

@@ -274,24 +274,33 @@ def test_linear_with_the_square_of_relu(dtype, M, N, K):
                                    (2100, 389 * 2, 160)])
 def test_linear_with_the_kernel_for_cta_pairs(M, N, K):
     """The product on pairs of CTAs (tcgen05 cta_group::2: tiles of 256 tokens x 256 weight rows, each
-    CTA loading half of the weight rows), which is off unless asked for: plain and with the SwiGLU
-    epilogue, with ragged last tiles on every side, bfloat16 and float32 results."""
+    CTA loading half of the weight rows) against the single-CTA kernel and against 64 bits: plain and with
+    the SwiGLU epilogue, with ragged last tiles on every side, bfloat16 and float32 results."""
+    import ctypes
     o = ops()
+
+    def on_pairs():
+        plan = (ctypes.c_int * 4)()
+        o.lib().zi_gemm_tcgen05_plan_for(M, N, K, 148, 74, plan)
+        return bool(plan[3])
+
     x = rnd(M, K, dtype=torch.bfloat16)
     w = rnd(N, K, dtype=torch.bfloat16, scale=0.05, seed=1)
     want = x.double() @ w.double().T
     before = o.gemm_pair_kernel(True)
     try:
+        assert on_pairs()
         got = o.linear(x, w)
         got32 = o.linear(x, w, out_dtype=torch.float32)
         if N % 128 == 0:
             wg, wu = w[:N // 2].contiguous(), w[N // 2:].contiguous()
             act = o.linear_swiglu(x, o.interleave_gate_up(wg, wu))
+        assert o.gemm_pair_kernel(False) is True and not on_pairs()
+        single = o.linear(x, w, out_dtype=torch.float32)
     finally:
         o.gemm_pair_kernel(before)
     torch.testing.assert_close(got.double(), want, rtol=8e-3, atol=1e-3)
     torch.testing.assert_close(got32.double(), want, rtol=1e-5, atol=1e-4)
-    single = o.linear(x, w, out_dtype=torch.float32)
     torch.testing.assert_close(got32, single, rtol=1e-5, atol=1e-4)
     if N % 128 == 0:
         g, u = want[:, :N // 2].float(), want[:, N // 2:].float()
@@ -869,9 +878,10 @@ def test_exact_attention_for_groups_of_heads_gives_the_plain_kernels_bits(nq, nk
         torch.testing.assert_close(got, ref.paged_attention(window=window, scale=scale, **args), **tol(torch.float32))
 
 
-@pytest.mark.parametrize("M,N,K", [(130, 4096, 4096), (300, 1024, 12288), (536, 4096, 12288), (257, 2050, 8200), (512, 12288, 512), (1024, 1280, 4160)])
-def test_products_that_the_rule_gives_to_cta_pairs(M, N, K):
-    """More than 128 tokens: the rule between the single-CTA kernel and CTA pairs, with and without a K split, plain, with
+@pytest.mark.parametrize("M,N,K", [(130, 4096, 4096), (300, 1024, 12288), (536, 4096, 12288), (257, 2050, 8200), (512, 12288, 512), (1024, 1280, 4160),
+                                   (384, 12288, 512)])
+def test_products_by_the_rule_for_cta_pairs(M, N, K):
+    """More than 128 tokens, on either side of the rule between the single-CTA kernel and CTA pairs: with and without a K split, plain, with
     the square of relu, as partial sums, with fresh weights (which pairs do not take) and gated."""
     o = ops()
     x = rnd(M, K, dtype=torch.bfloat16)

@@ -105,7 +105,7 @@ int zi_gemm_tcgen05_grouped(void* out, int out_dtype, const void* x, const void*
 int zi_gemm_tcgen05_heads(void* out, int out_dtype, const void* x, const void* w, int M, int N, int K, int ldx, int ldw,
                           int ldo, int groups, int x_group_cols, int out_group_cols, int sm_count, cudaStream_t stream);
 int zi_gemm_tcgen05_status();
-int zi_gemm_tcgen05_pair_enable(int on);
+int zi_gemm_tcgen05_pair_enable(int mode);
 
 int zi_paged_attention_tile_rows();
 int zi_paged_attention(void* out, int out_stride, const void* q, int q_stride, int dtype, const void* kcache,

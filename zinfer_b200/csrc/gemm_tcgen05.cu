@@ -811,10 +811,18 @@ static void plan_single(int M, int N, int K, int sm_count, int* plan) {
 }
 
 namespace {
-// Which kernel takes products of more than 128 tokens: -1 ask the environment (ZINFER_B200_GEMM_PAIR: 1 always the one for CTA
-// pairs where it can, 0 never), PAIR_AUTO the one that the rule below expects to be faster.
+// Which kernel takes products of more than 128 tokens: -1 ask the environment (ZINFER_B200_GEMM_PAIR: 1 and 0 as below),
+// PAIR_ALWAYS the one for CTA pairs for all of 256 tokens and more whose single-CTA plan has 256-wide tiles and no K split and
+// that fill the pairs' tiles, PAIR_AUTO the one that the rule below expects to be faster.
 constexpr int PAIR_NEVER = 0, PAIR_ALWAYS = 1, PAIR_AUTO = 2;
 int g_pair_mode = -1;
+int pair_mode() {
+  if (g_pair_mode < 0) {
+    const char* e = getenv("ZINFER_B200_GEMM_PAIR");
+    g_pair_mode = e && e[0] == '1' ? PAIR_ALWAYS : (e && e[0] == '0' ? PAIR_NEVER : PAIR_AUTO);
+  }
+  return g_pair_mode;
+}
 
 // The kernel for CTA pairs, or not, and its K splits.  Time in whole rounds of tiles: a k-block of a single CTA's 128 x 256
 // (or 128 x 128) tile takes 0.37 (0.31) us, of a pair's 256 x 256 tile 0.335 us (measured on full rounds of real weights; with
@@ -823,12 +831,9 @@ int g_pair_mode = -1;
 // 4096 282 -> 265, 2048 x 4096 x 12288 156 -> 144, 1024 x 4096 x 12288 80 -> 74, 512 x 24576 x 4096 89 -> 80.  `slots`: pairs
 // resident at once (resident_pairs).
 bool plan_pair(int M, int N, int K, int sm_count, int slots, int* plan) {
-  if (g_pair_mode < 0) {
-    const char* e = getenv("ZINFER_B200_GEMM_PAIR");
-    g_pair_mode = e && e[0] == '1' ? PAIR_ALWAYS : (e && e[0] == '0' ? PAIR_NEVER : PAIR_AUTO);
-  }
-  if (g_pair_mode == PAIR_NEVER || plan[0] || N < PAIR_TILE || slots <= 0) return false;
-  if (g_pair_mode == PAIR_ALWAYS) {
+  const int mode = pair_mode();
+  if (mode == PAIR_NEVER || plan[0] || N < PAIR_TILE || slots <= 0) return false;
+  if (mode == PAIR_ALWAYS) {
     // as far as it wastes little: 300 tokens would fill 512 rows of pair tiles but 384 of single tiles
     const int pair_rows = (M + PAIR_TILE - 1) / PAIR_TILE * PAIR_TILE, single_rows = (M + TILE_A - 1) / TILE_A * TILE_A;
     return plan[1] == PAIR_TILE && plan[2] == 1 && (pair_rows == single_rows || M >= 1024);
@@ -1179,11 +1184,11 @@ extern "C" int zi_gemm_tcgen05_argmax(float* out, const void* x, const void* w, 
                      EPI_ARGMAX, cand_val, cand_idx);
 }
 
-// Switches the kernel for CTA pairs on (1) for products of 256 tokens and more that fill its tiles, or back to the rule
-// that chooses (0); returns the setting before.
-extern "C" int zi_gemm_tcgen05_pair_enable(int on) {
-  const int before = g_pair_mode == PAIR_ALWAYS ? 1 : 0;
-  g_pair_mode = on ? PAIR_ALWAYS : PAIR_AUTO;
+// Sets whether products go to the kernel for CTA pairs: 0 never, 1 all that fill its tiles, 2 by the rule; returns the setting
+// before (the environment's, when nothing was set).
+extern "C" int zi_gemm_tcgen05_pair_enable(int mode) {
+  const int before = pair_mode();
+  g_pair_mode = mode < PAIR_NEVER || mode > PAIR_AUTO ? PAIR_AUTO : mode;
   return before;
 }
 

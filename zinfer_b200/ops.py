@@ -74,12 +74,13 @@ def selftest_waits_of_a_warp(device, code: int = 77, tries: int = 4096) -> torch
     return out
 
 
-def gemm_pair_kernel(on: bool) -> bool:
+def gemm_pair_kernel(on: Optional[bool]) -> Optional[bool]:
     """Switches the matrix product's kernel for CTA pairs (tcgen05 ``cta_group::2``: two SMs on one
     tile of 256 tokens x 256 weight rows, each loading half of the weight rows) on for all products of
-    256 tokens and more that fill its tiles, or back to the rule that chooses between the kernels
-    (``ZINFER_B200_GEMM_PAIR``: 1 as here, 0 never, else the rule); returns the setting before."""
-    return bool(lib().zi_gemm_tcgen05_pair_enable(1 if on else 0))
+    256 tokens and more that fill its tiles (True; those alone), off (False), or leaves the choice to the rule that weighs
+    both kernels (None, unless ``ZINFER_B200_GEMM_PAIR`` is 1 or 0); returns the setting before, to be handed back."""
+    before = int(lib().zi_gemm_tcgen05_pair_enable(2 if on is None else 1 if on else 0))
+    return None if before == 2 else before == 1
 
 
 def library_file() -> str:
