@@ -1,0 +1,62 @@
+"""What the operations tell their kernels about operands that may be read before the wait for earlier kernels: only what the
+caller has said is no output of this step.  The kernels are replaced by a recorder, so nothing here needs a GPU."""
+import pytest
+import torch
+
+from zinfer_b200 import ops
+
+
+class Recorder:
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.calls.append((name, args))
+            return 0
+        return call
+
+
+@pytest.fixture
+def recorder(monkeypatch):
+    r = Recorder()
+    monkeypatch.setattr(ops, "lib", lambda: r)
+    monkeypatch.setattr(ops, "_stream", lambda: None)
+    monkeypatch.setattr(ops, "_ptr", lambda t: None)
+    return r
+
+
+def early(recorder, name):
+    (args,) = [a for n, a in recorder.calls if n == name]
+    recorder.calls.clear()
+    return args[-2]
+
+
+def test_32_bit_products_read_weights_early_only_when_told(recorder):
+    x, w = torch.zeros(3, 8), torch.zeros(4, 8)
+    for said, want in ((None, 0), (True, 0), (False, 1)):
+        ops.linear(x, w, fresh_weight=said)
+        assert early(recorder, "zi_gemm_simt") == want
+    ops.linear(x, w)
+    assert early(recorder, "zi_gemm_simt") == 0
+    ops.linear_swiglu(x, torch.zeros(256, 8))
+    assert early(recorder, "zi_gemm_simt") == 0
+    ops.linear_argmax(x, w)
+    assert early(recorder, "zi_gemm_simt") == 0
+
+
+def test_models_say_that_their_weights_are_weights():
+    """Every product of a part with a bound weight by way of ``ops.linear`` says that it is one."""
+    import glob
+    import os
+    import re
+
+    for f in glob.glob(os.path.join(os.path.dirname(ops.__file__), "parts", "*.py")):
+        with open(f) as fh:
+            src = fh.read()
+        for m in re.finditer(r"ops\.linear\(", src):
+            depth, j = 1, m.end()
+            while depth:
+                depth += {"(": 1, ")": -1}.get(src[j], 0)
+                j += 1
+            assert src[m.start():j].endswith("fresh_weight=False)"), (os.path.basename(f), src[m.start():j])

@@ -765,15 +765,16 @@ def _sm_count(device: torch.device) -> int:
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
-           out: Optional[torch.Tensor] = None, allow_partials: bool = False, fresh_weight: bool = False,
+           out: Optional[torch.Tensor] = None, allow_partials: bool = False, fresh_weight: Optional[bool] = None,
            relu2: bool = False):
     """``x [M, K] @ weight [N, K]^T`` with 32-bit accumulation; with ``relu2`` the square of the product's relu
     (taken on the 32-bit sums: in the tensor-core product's epilogue, or where its K splits are added).
 
     With ``allow_partials`` a product that was split along K may come back as
     :class:`Partials` (its consumer adds the splits) instead of a tensor.  ``fresh_weight``:
-    ``weight`` is no weight but the output of an earlier kernel of this step (the tensor-core kernel and the
-    32-bit tiles otherwise request their first weight tiles before they wait for the kernels before them).
+    whether ``weight`` is no weight but the output of an earlier kernel of this step.  Where it is not, the kernels
+    request their first weight tiles before they wait for the kernels before them.  Without a word (None) the
+    tensor-core kernel takes ``weight`` for a weight, the 32-bit tiles wait.
 
     bfloat16 operands that meet TMA's alignment rules go to the tcgen05 kernel; float32
     operands (the true 32-bit path), mixed types and unaligned shapes go to the
@@ -805,7 +806,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     _need(out.stride(1) == 1, "linear: output rows must be dense")
     with _prof.region(f"linear (CUDA cores) N={N} K={K}", lambda: _nb(weight, out) + M * K * x.element_size(), 2 * M * N * K):
         _check(lib().zi_gemm_simt(_ptr(out), _tag(out), _ptr(x), _tag(x), _ptr(weight), _tag(weight), M, N, K,
-                                  x.stride(0), weight.stride(0), out.stride(0), 0 if fresh_weight else 1, _stream()), "linear")
+                                  x.stride(0), weight.stride(0), out.stride(0), 1 if fresh_weight is False else 0, _stream()), "linear")
     if relu2:
         _need(out.is_contiguous(), "linear: the square of relu wants dense results")
         relu2_(out)

@@ -270,7 +270,7 @@ class GQAttention(Mixer):
         if cache.writes and not self.projects_kv:
             raise ValueError("a mixer without key and value projections cannot be the one that fills its cache")
         w = self.w_qkv if cache.writes else self.w_qkv[:q_width]
-        qkv = ops.linear(x, w, out_dtype=self.ctx.dtype)
+        qkv = ops.linear(x, w, out_dtype=self.ctx.dtype, fresh_weight=False)
         group = step.kv_groups[cache.group]
         cos, sin = self.position.tables() if self.position is not None else (None, None)
         q = ops.qk_prepare(qkv, self.nq, self.nkv, self.d, self.rot_dims, self.q_norm, self.k_norm,
@@ -283,7 +283,7 @@ class GQAttention(Mixer):
 
     def _forward_rows(self, x, step, cache):
         # 32-bit results of the product: the biases and the norm over the whole row meet the unrounded sums
-        proj = ops.linear(x, self.w_rows, out_dtype=torch.float32)
+        proj = ops.linear(x, self.w_rows, out_dtype=torch.float32, fresh_weight=False)
         group = step.kv_groups[cache.group]
         cos, sin = self.position.tables() if self.position is not None else (None, None)
         q, gate = ops.qkv_rows_prepare(proj, self.row_bias, self.nq, self.nkv, self.d, self.dv, self.n_gate, self.q_norm,
@@ -294,7 +294,7 @@ class GQAttention(Mixer):
                               dist_bias=self.dist_table)
         if gate is not None:
             heads = ops.sigmoid_gate(heads, gate, out=heads, group=self.dv if self.output_gate == "head" else 1)
-        return ops.linear(heads, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+        return ops.linear(heads, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
 
     def _forward_conv(self, x, step, cache):
         conv = None
@@ -303,7 +303,7 @@ class GQAttention(Mixer):
         if not cache.writes:
             raise ValueError("the conv form of attention fills its own cache")
         # 32-bit results of the product: the biases and the convolution meet the unrounded sums
-        proj = ops.linear(x, self.w_rows, out_dtype=torch.float32, allow_partials=True)
+        proj = ops.linear(x, self.w_rows, out_dtype=torch.float32, allow_partials=True, fresh_weight=False)
         group = step.kv_groups[cache.group]
         tables = self.position.tables() if self.position is not None else (None, None)
         q = torch.empty((x.shape[0], self.nq * self.d), dtype=self.ctx.dtype, device=x.device)
@@ -316,7 +316,7 @@ class GQAttention(Mixer):
         heads = ops.attention(q, cache.k, cache.v, group.block_tables, step, self.nq, self.nkv, self.d, cache.page_size,
                               self.window, self.scale, value_dim=self.dv, sink_logit=self.sink_logit, softcap=self.softcap,
                               dist_bias=self.dist_table)
-        return ops.linear(heads, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+        return ops.linear(heads, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
 
     VALUES_CARRIED = "first values"      # under this name the first mixing layer hands its values on
 
@@ -327,7 +327,7 @@ class GQAttention(Mixer):
         if not cache.writes:
             raise ValueError("the heads form of attention fills its own cache")
         # 32-bit results of the product: biases, norms and the mix of values meet the unrounded sums
-        proj = ops.linear(x, self.w_qkv, out_dtype=torch.float32, allow_partials=True)
+        proj = ops.linear(x, self.w_qkv, out_dtype=torch.float32, allow_partials=True, fresh_weight=False)
         group = step.kv_groups[cache.group]
         cos, sin = self.position.tables() if self.position is not None else (None, None)
         first = bool(self.value_mix and self.value_mix.get("first"))
@@ -345,7 +345,7 @@ class GQAttention(Mixer):
             ops.pool_blocks(cache.k, cache.v, group.block_tables, pooled, pgroup.slot_mapping, step, cache.page_size)
         heads = ops.attention(q, cache.k, cache.v, group.block_tables, step, self.nq, self.nkv, self.d, cache.page_size, self.window,
                               self.scale, sink=self.sink, value_dim=self.dv, pooled=pooled)
-        return ops.linear(heads, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+        return ops.linear(heads, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
 
     def forward(self, x, step, cache):
         if self.conv_form:
@@ -357,10 +357,10 @@ class GQAttention(Mixer):
                 raise ValueError("the rows form of attention fills its own cache")
             return self._forward_rows(x, step, cache)
         if self.general:
-            return ops.linear(self.heads_out(x, step, cache), self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+            return ops.linear(self.heads_out(x, step, cache), self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
         q_width = self.nq * self.d
         w = self.w_qkv if cache.writes else self.w_qkv[:q_width]  # a reader of another's cache needs q only
-        qkv = ops.linear(x, w, out_dtype=self.ctx.dtype, allow_partials=True)
+        qkv = ops.linear(x, w, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
         group = step.kv_groups[cache.group]
         cos, sin = self.position.tables() if self.position is not None else (None, None)
         if cache.writes and ops.decode_fused_ok(self.ctx.dtype, self.nq, self.nkv, self.d, step):
@@ -369,14 +369,14 @@ class GQAttention(Mixer):
                 qkv, self.nq, self.nkv, self.d, self.q_norm, self.k_norm,
                 self.qk_norm_eps if self.qk_norm_eps is not None else 0.0, cos, sin, cache.k, cache.v,
                 group.slot_mapping, group.block_tables, step, cache.page_size, self.window, self.scale)
-            return ops.linear(o, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+            return ops.linear(o, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
         q = ops.qk_norm_rope_store(
             qkv, self.nq, self.nkv, self.d, self.q_norm, self.k_norm,
             self.qk_norm_eps if self.qk_norm_eps is not None else 0.0, cos, sin, step.positions,
             cache.k, cache.v, group.slot_mapping, cache.page_size, write_kv=cache.writes, out_dtype=self.ctx.dtype)
         o = ops.attention(q, cache.k, cache.v, group.block_tables, step, self.nq, self.nkv, self.d,
                           cache.page_size, self.window, self.scale)
-        return ops.linear(o, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+        return ops.linear(o, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
 
 
 def distance_buckets(rows: int, far: float) -> list[int]:

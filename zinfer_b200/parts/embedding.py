@@ -98,7 +98,7 @@ class LMHead(Part):
         self.weight = table
 
     def forward(self, x):
-        logits = ops.linear(x, self.weight, out_dtype=torch.float32)
+        logits = ops.linear(x, self.weight, out_dtype=torch.float32, fresh_weight=False)
         return logits if self.scale == 1.0 else ops.scale_(logits, self.scale)
 
     def forward_argmax(self, x):

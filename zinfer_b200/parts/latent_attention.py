@@ -111,7 +111,7 @@ class LatentAttention(Mixer):
         if x.shape[0] > self.PER_HEAD_TENSOR_FROM and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 \
                 and ops.tensor_core_linear_ok(x[:, 0], weight[0]) and ops.tensor_core_linear_ok(x[:, -1], weight[-1]):
             for n in range(self.heads):
-                ops.linear(x[:, n], weight[n], out=out[:, n])
+                ops.linear(x[:, n], weight[n], out=out[:, n], fresh_weight=False)
         else:
             ops.linear_batched(x.transpose(0, 1), weight, out.transpose(0, 1))
         return out
@@ -125,15 +125,15 @@ class LatentAttention(Mixer):
         if self.q_rank:
             # queries through their own latent: [W_dq; W_dkv; W_g] h with 32-bit results (both norms meet the unrounded
             # sums), the norm of the query latent, W_uq
-            proj = ops.linear(x, self.w_in, out_dtype=torch.float32)
+            proj = ops.linear(x, self.w_in, out_dtype=torch.float32, fresh_weight=False)
             qs = ops.linear(ops.rmsnorm_rows(proj[:, :self.q_rank], self.q_norm, self.eps, self.ctx.dtype), self.w_uq,
-                            out_dtype=self.ctx.dtype)
+                            out_dtype=self.ctx.dtype, fresh_weight=False)
             ops.latent_prepare_rows(qs, proj[:, self.q_rank:], H, self.dim, self.rot_dim, self.rank, self.rot_dims,
                                     self.neighbours, self.c_norm, self.eps, cos, sin, step.positions, q_eff,
                                     cache.k if cache.writes else None, group.slot_mapping)
             gate_at = self.q_rank + D
         else:
-            proj = qs = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype)
+            proj = qs = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype, fresh_weight=False)
             if self.neighbours:
                 ops.latent_prepare_rows(proj, proj[:, qw:], H, self.dim, self.rot_dim, self.rank, self.rot_dims, True,
                                         self.c_norm, self.eps, cos, sin, step.positions, q_eff,
@@ -152,4 +152,4 @@ class LatentAttention(Mixer):
         if self.gated:
             gate = proj[:, gate_at:gate_at + H * self.vdim]
             heads = ops.sigmoid_gate(heads, gate if gate.dtype == heads.dtype else gate.to(heads.dtype), out=heads)
-        return ops.linear(heads, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+        return ops.linear(heads, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)

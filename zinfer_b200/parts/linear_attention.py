@@ -83,13 +83,13 @@ class GatedLinearAttention(Mixer):
 
     def forward(self, x, step, cache):
         qk, hv = self.heads * self.dim, self.heads * self.vdim
-        proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype)
+        proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype, fresh_weight=False)
         q, k, v, g = proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:2 * qk + hv], proj[:, 2 * qk + hv:2 * qk + 2 * hv]
         decay = ops.low_rank_decay(proj[:, 2 * qk + 2 * hv:], self.w_a2, self.a_bias, None, self.tau, self.dim)
         o = ops.channel_decay_recurrence(q, k, v, decay, None, self.dim ** -0.5, cache.state, self.heads, self.heads, self.dim, self.vdim, step,
                                          fast=self.ctx.dtype == torch.bfloat16)
         y = ops.head_norm_gate(o, self.norm, self.eps, g, "silu", self.heads, self.vdim, self.ctx.dtype)
-        return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+        return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
 
 
 class HGRN2(Mixer):
@@ -124,10 +124,10 @@ class HGRN2(Mixer):
 
     def forward(self, x, step, cache):
         # 32-bit results of the product: the gate and the recurrence read the unrounded sums (and add its K splits)
-        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, allow_partials=True)
+        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, allow_partials=True, fresh_weight=False)
         y = ops.linear_recurrence_gated(proj, self.lower, self.f_bias, cache.state, self.heads, self.dim, self.vdim, step,
                                         norm_weight=self.norm, norm_eps=self.eps, out_dtype=self.ctx.dtype)
-        return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+        return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
 
 
 class GatedDeltaRule(Mixer):
@@ -206,7 +206,7 @@ class GatedDeltaRule(Mixer):
 
     def _forward_head_decay(self, x, step, state):
         C, H, qk, hv = self.channels, self.heads, self.qk, self.hv
-        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, allow_partials=True)
+        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, allow_partials=True, fresh_weight=False)
         cols = lambda at, n: ops.Columns(proj, at, n)
         tail = state[:, self.s_size:].view(state.shape[0], self.taps - 1, C)
         qkv = torch.empty((x.shape[0], C), dtype=torch.float32, device=x.device)
@@ -218,13 +218,13 @@ class GatedDeltaRule(Mixer):
             decay=("delta", cols(C + hv, H), cols(C + hv + H, H), self.a_log, self.dt_bias))
         y = ops.head_decay_recurrence(q, k, v, decay, beta, state[:, :self.s_size], H, self.kv_heads, self.dim, self.vdim, step, delta=True,
                                       fast=self.ctx.dtype == torch.bfloat16, norm=(self.norm, self.eps, cols(C, hv), self.ctx.dtype))
-        return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+        return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
 
     def forward(self, x, step, cache):
         if self.head_decay:
             return self._forward_head_decay(x, step, cache.state)
         C, H, qk = self.channels, self.heads, self.qk
-        proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype)
+        proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype, fresh_weight=False)
         state = cache.state
         s_view = state[:, :self.s_size]
         tail = state[:, self.s_size:].view(state.shape[0], self.taps - 1, C)
@@ -238,9 +238,9 @@ class GatedDeltaRule(Mixer):
         decay = ops.low_rank_decay(proj[:, a0:a0 + self.decay_rank], self.w_a2, self.dt_bias, self.a_log, 1.0, self.dim)
         o = ops.channel_decay_recurrence(q, k, v, decay, beta, self.dim ** -0.5, s_view, H, self.kv_heads, self.dim, self.vdim, step,
                                          fast=self.ctx.dtype == torch.bfloat16)
-        gate = ops.linear(proj[:, a0 + self.decay_rank:], self.w_g2, out_dtype=self.ctx.dtype)
+        gate = ops.linear(proj[:, a0 + self.decay_rank:], self.w_g2, out_dtype=self.ctx.dtype, fresh_weight=False)
         y = ops.head_norm_gate(o, self.norm, self.eps, gate, "sigmoid", H, self.vdim, self.ctx.dtype)
-        return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+        return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
 
 
 class ParallelMixer(Mixer):

@@ -71,7 +71,7 @@ class Mamba2(Mixer):
     def forward(self, x, step, cache):
         C, H, inner, bc = self.channels, self.heads, self.inner, self.bc
         state = cache.state
-        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, allow_partials=True)
+        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, allow_partials=True, fresh_weight=False)
         cols = lambda at, n: ops.Columns(proj, at, n)
         tail = state[:, self.s_size:].view(state.shape[0], self.taps - 1, C)
         xbc = torch.empty((x.shape[0], C), dtype=torch.float32, device=x.device)
@@ -82,4 +82,4 @@ class Mamba2(Mixer):
                                       fast=self.ctx.dtype == torch.bfloat16)
         y = ops.gated_part_norm(y, cols(0, inner), self.norm, self.eps, self.norm_groups, self.ctx.dtype, skip=self.skip, x=xs,
                                 vdim=self.vdim)
-        return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+        return ops.linear(y, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)

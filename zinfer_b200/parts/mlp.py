@@ -51,13 +51,13 @@ class SwiGLUMLP(FeedForward):
         if self.interleaved:
             act = ops.linear_swiglu(x, self.w_gate_up, out_dtype=self.ctx.dtype, activation=self.activation)
         else:
-            gu = ops.linear(x, self.w_gate_up, out_dtype=self.ctx.dtype, allow_partials=True)
+            gu = ops.linear(x, self.w_gate_up, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
             if self.clamped:
                 act = ops.clamped_gate(gu, self.limit, self.act_alpha, 1.0, self.ctx.dtype)
             else:
                 act = ops.swiglu(gu, out_dtype=self.ctx.dtype, activation=self.activation)
         # the product may come back as split-K partial sums; the next norm adds them with the residual
-        return ops.linear(act, self.w_down, out_dtype=self.ctx.dtype, allow_partials=True)
+        return ops.linear(act, self.w_down, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
 
 
 class PlainMLP(FeedForward):
@@ -82,5 +82,5 @@ class PlainMLP(FeedForward):
         self.w_down = tensors[self.names[1]].contiguous()
 
     def forward(self, x):
-        mid = ops.linear(x, self.w_up, out_dtype=self.ctx.dtype, relu2=True)
-        return ops.linear(mid, self.w_down, out_dtype=self.ctx.dtype, allow_partials=True)
+        mid = ops.linear(x, self.w_up, out_dtype=self.ctx.dtype, relu2=True, fresh_weight=False)
+        return ops.linear(mid, self.w_down, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)

@@ -72,16 +72,16 @@ class RGLRUMixer(Mixer):
 
     def forward(self, x, step, cache):
         T, W, B, bw = x.shape[0], self.width, self.blocks, self.bw
-        yx = ops.linear(x, self.w_yx, out_dtype=self.ctx.dtype)         # [T, 2W]: y branch, then x branch
+        yx = ops.linear(x, self.w_yx, out_dtype=self.ctx.dtype, fresh_weight=False)         # [T, 2W]: y branch, then x branch
         if step.all_decode and step.n_seqs == T:
             # one token per request: convolution, gates and recurrence are one kernel
             mixed = ops.rglru_decode(yx, self.y_bias, self.x_bias, self.conv, self.conv_bias, self.w_gates, self.r_bias,
                                      self.i_bias, self.lam, self.decay_scale, cache.state, step)
-            return ops.linear(mixed, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+            return ops.linear(mixed, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
         y, xb = yx[:, :W], yx[:, W:]
         u = ops.causal_conv(xb, self.x_bias, self.conv, self.conv_bias, cache.state, step)     # float32 [T, W]
         gates = torch.empty((T, B, 2 * bw), dtype=torch.float32, device=x.device)
         ops.linear_batched(u.view(T, B, bw).transpose(0, 1), self.w_gates, gates.transpose(0, 1))
         mixed = ops.rglru_scan(u, gates, bw, self.r_bias, self.i_bias, self.lam, self.decay_scale, y, self.y_bias,
                                xb, self.x_bias, cache.state, step)
-        return ops.linear(mixed, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True)
+        return ops.linear(mixed, self.w_o, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
