@@ -45,6 +45,18 @@ def test_32_bit_products_read_weights_early_only_when_told(recorder):
     assert early(recorder, "zi_gemm_simt") == 0
 
 
+def test_norms_of_updates_and_decays_read_nothing_before_their_wait():
+    """In the kernels themselves: the wait for earlier kernels stands before the first read of an operand."""
+    import os
+    import re
+
+    for f, kernel in (("elementwise.cu", "norm_residual_few_kernel"), ("linear_attention.cu", "low_rank_decay_kernel")):
+        with open(os.path.join(os.path.dirname(ops.__file__), "csrc", f)) as fh:
+            body = fh.read().split(kernel + "(", 1)[1].split("{", 1)[1]
+        before = body[:body.index("pdl_wait();")]
+        assert not re.search(r"\b(w|bias|a_log|x|h|a|ap|b|bp)\s*\[|load\(", before), kernel
+
+
 def test_models_say_that_their_weights_are_weights():
     """Every product of a part with a bound weight by way of ``ops.linear`` says that it is one."""
     import glob

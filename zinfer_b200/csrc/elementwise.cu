@@ -1383,13 +1383,13 @@ norm_residual_few_kernel(float* __restrict__ h, const TA* __restrict__ a, const 
   pdl_launch_dependents();
   __shared__ float scratch[33];
   const size_t row = (size_t)blockIdx.x * H;
+  pdl_wait();
   float4 ww[VPT], y[VPT], x[VPT];
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {                      // the norm's weights do not depend on the kernel before this one
+  for (int i = 0; i < VPT; ++i) {
     const int c = 4 * (threadIdx.x + i * blockDim.x);
     ww[i] = c < H ? Vec4<float>::load(w + c) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  pdl_wait();
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {

@@ -103,11 +103,11 @@ low_rank_decay_kernel(float* __restrict__ out, const __nv_bfloat16* __restrict__
                       int T, int N, int D, int tokens, const float* __restrict__ bias, const float* __restrict__ a_log, float inv_tau) {
   pdl_launch_dependents();
   const int c = blockIdx.x * blockDim.x + threadIdx.x, t0 = blockIdx.y * tokens;
-  float wr[R];                                       // weights do not depend on the kernel before this one
+  pdl_wait();
+  float wr[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) wr[r] = c < N && r < rank ? to_f32(w[(size_t)c * rank + r]) : 0.f;
   const float add = c < N && bias ? bias[c] : 0.f, rate = c < N && a_log ? expf(a_log[c / D]) : 0.f;
-  pdl_wait();
   if (c >= N) return;
   const int t1 = min(T, t0 + tokens);
   for (int t = t0; t < t1; ++t) {
