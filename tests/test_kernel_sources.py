@@ -28,3 +28,16 @@ def test_no_lane_leaves_its_warp_on_its_own_answer():
             if f not in ("tcgen05_ptx.cuh", "gemm_f32_tiles.cuh"):
                 assert not re.search(r"(?<![A-Za-z_])mbar_wait\([^;{]*\)\s*\{[^}]*\b(break|return)\b", src), f
     assert found == alone
+
+
+def test_every_wait_that_runs_out_names_its_kernel():
+    """Status codes belong to one kind of kernel each, and the error says which."""
+    from zinfer_b200 import ops
+
+    of = {"attention_tcgen05.cu": "the attention", "attention_tiles.cuh": "the attention", "gemm_f32_tiles.cuh": "the 32-bit product of few rows",
+          "gemm_tcgen05.cu": "the tensor-core product"}
+    for f, name in of.items():
+        with open(os.path.join(CSRC, f)) as fh:
+            src = fh.read()
+        codes = [int(c) for c in re.findall(r"atomicExch\(status, (\d+)\)|status, (\d+), \[&\]", src) for c in c if c]
+        assert codes and all(ops.waiting_kernel(c).startswith(name) for c in codes), (f, codes)

@@ -264,7 +264,7 @@ gemm_f32_few_kernel(TO* __restrict__ out, const float* __restrict__ x, const flo
       copy_x(c);
     }
     if (failed) {                          // copies in flight land before shared memory is given up
-      atomicExch(status, 21);
+      atomicExch(status, 31);
       for (int i = 0; i < 64; ++i) __nanosleep(10000);
     }
     return;
@@ -289,7 +289,7 @@ gemm_f32_few_kernel(TO* __restrict__ out, const float* __restrict__ x, const flo
     if (lane == 0) mbar_arrive(&empty[s]);
   }
   if (failed) {
-    atomicExch(status, 22);
+    atomicExch(status, 32);
     for (int i = 0; i < 64; ++i) __nanosleep(10000);
     return;
   }

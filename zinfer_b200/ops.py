@@ -45,18 +45,27 @@ def lib() -> ctypes.CDLL:
 
 
 def kernel_status() -> int:
-    """Reads and clears the status words of the tcgen05 kernels (synchronises).
-    0: every bounded wait inside them completed; else the code of the wait that ran out."""
-    return int(lib().zi_gemm_tcgen05_status())   # one word for the products and the tcgen05 attention
+    """Reads and clears the word in which kernels record bounded waits that ran out (synchronises).
+    0: every one completed; else the code of the wait that ran out (:func:`waiting_kernel` says whose)."""
+    return int(lib().zi_gemm_tcgen05_status())   # one word for the products and the attention
+
+
+def waiting_kernel(code: int) -> str:
+    """The kernel whose wait a status code stands for."""
+    for first, last, name in ((1, 4, "the tensor-core product"), (5, 8, "the tensor-core product on CTA pairs"), (11, 21, "the attention"),
+                              (31, 32, "the 32-bit product of few rows")):
+        if first <= code <= last:
+            return name
+    return "a kernel"
 
 
 def require_kernel_status_ok(where: str) -> None:
-    """Raises if a bounded wait inside a tensor-core kernel ran out since the last check (its
+    """Raises if a bounded wait inside a kernel ran out since the last check (its
     results are then not to be trusted).  Synchronises; the engine calls it where it waits for
     the device anyway, and every so many steps."""
     code = kernel_status()
     if code != 0:
-        raise KernelError(f"{where}: a wait inside a tensor-core kernel ran out (code {code}); its results are invalid")
+        raise KernelError(f"{where}: a wait inside {waiting_kernel(code)} ran out (code {code}); its results are invalid")
 
 
 def selftest_wait_runs_out(code: int = 77, tries: int = 4096) -> None:
