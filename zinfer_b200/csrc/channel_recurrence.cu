@@ -27,8 +27,8 @@
 // not survive the split into parts.  So a block of the walk whose outputs or state come out so takes its request, head and
 // value channels again token by token from the state it began with (walk_tokens), as the recurrence is written.
 //
-// A chunk's place in the workspace: request s's chunk i lies at cu_q[s] / 64 + s + i, so that no prefix sum over the
-// requests is needed.  Requests that bring one token are left alone.
+// A chunk's place in the workspace: the chunks of the requests that bring two tokens or more, one behind the other.  Requests
+// that bring one token are left alone and have no place.
 //
 // Measured, 2,048 tokens, 8 heads of 128 x 256 (the walk token by token -> chunks): plain form with bfloat16 q, k, v 756 -> 171 us,
 // delta rule 833 -> 242 us.  Of that (one kernel at a time) the scores 39 and 50 us, the triangular systems 45, the walk 155.
@@ -55,7 +55,7 @@ struct ChannelJob {
   int H, G, D, V;
   const int* cu_q;
   const int* state_slots;
-  int n_seqs;
+  int n_seqs, places;  // places: for whose chunks the workspace has room
   float* out;          // [T][H * V]
   int ldo;
   // workspace, per place and head
@@ -68,16 +68,42 @@ struct ChannelJob {
   float* u0;           // [RK][V]  delta rule only
 };
 
+__device__ __forceinline__ int chunks_of(int qlen) { return qlen > 1 ? (qlen + RK - 1) / RK : 0; }
+
+// The request and chunk at a place, by a whole warp: 32 requests at a time, their chunks counted together.
 __device__ __forceinline__ bool channel_chunk(const ChannelJob& j, int place, int& first, int& n) {
-  int lo = 0, hi = j.n_seqs - 1;      // the last request whose first place is at or before this one
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (j.cu_q[mid] / RK + mid <= place) lo = mid; else hi = mid - 1;
+  const int lane = threadIdx.x & 31;
+  int before = 0;
+  for (int s0 = 0; s0 < j.n_seqs; s0 += 32) {
+    const int s = s0 + lane;
+    int tok0 = 0, qlen = 0;
+    if (s < j.n_seqs) {
+      tok0 = j.cu_q[s];
+      qlen = j.cu_q[s + 1] - tok0;
+    }
+    const int own = chunks_of(qlen);
+    int upto = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += y;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, place < before + upto);
+    if (hit) {
+      const int src = __ffs(hit) - 1, i = place - before - __shfl_sync(0xffffffffu, upto - own, src);
+      first = __shfl_sync(0xffffffffu, tok0, src) + i * RK;
+      n = min(RK, __shfl_sync(0xffffffffu, qlen, src) - i * RK);
+      return true;
+    }
+    before += __shfl_sync(0xffffffffu, upto, 31);
   }
-  const int tok0 = j.cu_q[lo], qlen = j.cu_q[lo + 1] - tok0, i = place - (tok0 / RK + lo);
-  first = tok0 + i * RK;
-  n = min(RK, qlen - i * RK);
-  return qlen > 1 && i >= 0 && n > 0;
+  return false;
+}
+// The place of a request's first chunk, by a whole warp.
+__device__ __forceinline__ int first_place(const ChannelJob& j, int seq) {
+  int before = 0;
+  for (int s = threadIdx.x & 31; s < seq; s += 32) before += chunks_of(j.cu_q[s + 1] - j.cu_q[s]);
+  return __reduce_add_sync(0xffffffffu, before);
 }
 
 constexpr int SP = RV + 8;                           // pitch of the state and of U: a fragment's reads fall into 32 banks
@@ -452,7 +478,8 @@ channel_walk_kernel(const __grid_constant__ ChannelJob j) {
   pdl_wait();
   const int tok0 = j.cu_q[seq], qlen = j.cu_q[seq + 1] - tok0;
   if (qlen <= 1) return;
-  const int chunks = (qlen + RK - 1) / RK, place0 = tok0 / RK + seq;
+  const int chunks = chunks_of(qlen), place0 = first_place(j, seq);
+  if (place0 + chunks > j.places) return;            // more such requests than the caller has counted: no room for their chunks
   float* state = j.state + (size_t)j.state_slots[seq] * j.slot_stride + (size_t)h * D * j.V;
   const int fr = lane >> 2, fk = lane & 3, fc = wc + fk * 2;      // a fragment's row, its channel of eight; a result's column
 
@@ -624,28 +651,33 @@ ChannelPlan channel_plan(int places, int H, int D, int V, int delta) {
 extern "C" int zi_channel_recurrence_supported(int D, int V, int H, int G) {
   return D >= 16 && D <= 128 && D % 16 == 0 && V > 0 && H > 0 && G > 0 && H % G == 0 && H <= 65535 && (V + RV - 1) / RV <= 65535;
 }
-extern "C" long long zi_channel_recurrence_workspace_floats(int T, int n_seqs, int H, int D, int V, int delta) {
-  return channel_plan(T / RK + n_seqs + 1, H, D, V, delta).total;
+// Chunks of the requests that bring two tokens or more, at most: n_single of the step's n_seqs requests bring one.
+static int channel_places(int T, int n_seqs, int n_single) { return (T - n_single) / RK + n_seqs - n_single; }
+
+extern "C" long long zi_channel_recurrence_workspace_floats(int T, int n_seqs, int n_single, int H, int D, int V, int delta) {
+  return channel_plan(channel_places(T, n_seqs, n_single), H, D, V, delta).total;
 }
 
-// The portions of two tokens and more of a step; requests that bring one token are left alone.  decay: float32 [T][H * D],
+// The portions of two tokens and more of a step; the n_single requests that bring one token are left alone.  decay: float32 [T][H * D],
 // between 0 and 1; beta: step sizes [T][H] or null (then without the delta rule); q and k of one type, v of its own;
 // workspace: zi_channel_recurrence_workspace_floats, 16-byte aligned.
 extern "C" int zi_channel_recurrence(float* out, int ldo, const void* q, int ldq, const void* k, int ldk, int qk_dtype, const void* v,
                                      int ldv, int v_dtype, const float* decay, int ldg, const float* beta, int ldb, float q_scale,
                                      float* state, long long slot_stride, int T, int H, int G, int D, int V, int delta, const int* cu_q,
-                                     const int* state_slots, int n_seqs, float* workspace, cudaStream_t stream) {
+                                     const int* state_slots, int n_seqs, int n_single, float* workspace, cudaStream_t stream) {
   if (T <= 0 || n_seqs <= 0) return 0;
+  if (n_single < 0 || n_single > n_seqs || n_single > T) return zi_refuse("channel_recurrence: %d of %d requests bring one token", n_single, n_seqs);
+  const int places = channel_places(T, n_seqs, n_single);
+  if (places == 0) return 0;
   if (!zi_channel_recurrence_supported(D, V, H, G)) return zi_refuse("channel_recurrence: %d heads (%d of keys) of %d x %d", H, G, D, V);
   if (!workspace || ((uintptr_t)workspace & 15) || !decay || (delta && !beta))
     return zi_refuse("channel_recurrence: needs decays, with the delta rule steps, and an aligned workspace");
-  const int places = T / RK + n_seqs + 1;
   const ChannelPlan p = channel_plan(places, H, D, V, delta);
   ChannelJob j = {};
   j.q = q; j.k = k; j.v = v; j.decay = decay; j.beta = beta;
   j.ldq = ldq; j.ldk = ldk; j.ldv = ldv; j.ldg = ldg; j.ldb = ldb; j.qk_dtype = qk_dtype; j.q_scale = q_scale;
   j.state = state; j.slot_stride = slot_stride; j.H = H; j.G = G; j.D = D; j.V = V;
-  j.cu_q = cu_q; j.state_slots = state_slots; j.n_seqs = n_seqs; j.out = out; j.ldo = ldo;
+  j.cu_q = cu_q; j.state_slots = state_slots; j.n_seqs = n_seqs; j.places = places; j.out = out; j.ldo = ldo;
   float* at = workspace;
   j.qd = at; at += p.rows;
   j.kd = at; at += p.rows;

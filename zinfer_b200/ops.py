@@ -1951,14 +1951,15 @@ def channel_decay_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
     _need(decay.dtype == torch.float32 and decay.stride(1) == 1 and tuple(decay.shape) == (T, heads * dim), "channel_decay_recurrence: decay")
     _need(not delta or (beta.dtype == torch.float32 and beta.stride(1) == 1 and tuple(beta.shape) == (T, heads)), "channel_decay_recurrence: beta")
     out = torch.empty((T, heads * vdim), dtype=torch.float32, device=q.device)
-    n = L.zi_channel_recurrence_workspace_floats(T, step.n_seqs, heads, dim, vdim, 1 if delta else 0)
+    n = L.zi_channel_recurrence_workspace_floats(T, step.n_seqs, step.n_dec, heads, dim, vdim, 1 if delta else 0)
     ws = torch.empty((n,), dtype=torch.float32, device=q.device)
     with _prof.region("recurrence in chunks, decays per channel" + (" (delta rule)" if delta else ""),
                       lambda: _nb(q, k, v, decay, out) + 2 * step.n_seqs * heads * dim * vdim * 4, 6 * T * heads * dim * vdim):
         _check(L.zi_channel_recurrence(
             _ptr(out), out.stride(0), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _tag(q), _ptr(v), v.stride(0), _tag(v), _ptr(decay),
             decay.stride(0), _ptr(beta), beta.stride(0) if delta else 0, ctypes.c_float(q_scale), _ptr(st), _ll(stride), T, heads, key_heads,
-            dim, vdim, 1 if delta else 0, _ptr(step.cu_q), _ptr(step.state_slots), step.n_seqs, _ptr(ws), _stream()), "channel_recurrence")
+            dim, vdim, 1 if delta else 0, _ptr(step.cu_q), _ptr(step.state_slots), step.n_seqs, step.n_dec, _ptr(ws), _stream()),
+            "channel_recurrence")
     if step.n_dec > 0:
         linear_recurrence(q, k, v, decay, beta, q_scale, state, heads, key_heads, dim, vdim, step, only_single=True, out=out)
     return out
