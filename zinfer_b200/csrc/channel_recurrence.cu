@@ -18,10 +18,10 @@
 //   1. channel_scores  per chunk and head: P, the products k . k, q and k times their decays
 //   2. channel_solve   (delta rule) per chunk and head: the triangular system by forward substitution, a thread per column
 //   3. channel_walk    per request, head and 16 value channels: the chunks in order, products with the state on the
-//                      tensor cores (mma.sync, tf32)
-// Everything is 32-bit: the tensor cores' operands are split into two tf32 parts (22 bits of mantissa; the product of the
-// two remainders is below the sums' rounding), the parts' products are summed apart, and the state is moved on by 32-bit
-// multiply-adds outside of the tensor cores' accumulators.  Against 64 bits outputs and states are as near as the walk's.
+//                      tensor cores (mma.sync, bfloat16 parts)
+// Everything is 32-bit: the tensor cores' operands are split into three bfloat16 parts (all 24 bits of mantissa), the parts'
+// products are summed apart, and the state is moved on by 32-bit multiply-adds outside of the tensor cores' accumulators.
+// Against 64 bits outputs and states are nearer than the walk's.
 //
 // A value that is infinite or no number would reach earlier tokens too (zero weights meet it in P U) and infinities would
 // not survive the split into parts.  So a block of the walk whose outputs or state come out so takes its request, head and
@@ -30,8 +30,10 @@
 // A chunk's place in the workspace: the chunks of the requests that bring two tokens or more, one behind the other.  Requests
 // that bring one token are left alone and have no place.
 //
-// Measured, 2,048 tokens, 8 heads of 128 x 256 (the walk token by token -> chunks): plain form with bfloat16 q, k, v 756 -> 171 us,
-// delta rule 833 -> 242 us.  Of that (one kernel at a time) the scores 39 and 50 us, the triangular systems 45, the walk 155.
+// Measured, 2,048 tokens, 8 heads of 128 x 256 (the walk token by token -> chunks): plain form with bfloat16 q, k, v 756 -> 182 us,
+// delta rule 833 -> 259 us.  Relative errors of outputs and states against 64 bits, 1e-7 (the walk -> chunks): plain 4.9, 5.8 ->
+// 3.3, 3.6, delta rule 2.1, 1.4 -> 1.6, 0.9.  (Two tf32 parts, 22 bits, and rows that took off their terms one by one: 168 and 242 us,
+// but 2.5, 1.7 with the delta rule, and plain at 8 x 64 tokens 1.65 against the walk's 1.52.)
 #include "api.h"
 #include "common.cuh"
 
@@ -106,24 +108,35 @@ __device__ __forceinline__ int first_place(const ChannelJob& j, int seq) {
   return __reduce_add_sync(0xffffffffu, before);
 }
 
-constexpr int SP = RV + 8;                           // pitch of the state and of U: a fragment's reads fall into 32 banks
+constexpr int SP = RV + 8;                           // pitch of the state and of U, pairs of rows: a fragment's reads fall into 32 banks
+constexpr int PP = RK + 8;                           // of P; Q and W have D + 8 (read as pairs along a row), K D + 4 (along a column)
 
-// The first part rounded to nearest by integer arithmetic (the conversion instruction has an eighth of its rate); the second
-// is what is left, of which the tensor cores read 11 bits.  A NaN stays one in the second part.
-__device__ __forceinline__ void tf32_parts(float x, uint32_t& hi, uint32_t& lo) {
-  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-  lo = __float_as_uint(x - __uint_as_float(hi));
+// Two values in three bfloat16 parts each, x in the low halves: 8 bits of mantissa rounded to nearest, then 8 of what is left, then
+// the rest, which is no more than 8.  The parts' sum is the value: all 24 bits are there.
+__device__ __forceinline__ uint32_t pack_nearest(float x, float y) {
+  uint32_t p;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p) : "f"(y), "f"(x));
+  return p;
 }
-__device__ __forceinline__ void tf32_mma(float (&d)[4], const uint32_t* a, const uint32_t* b) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+__device__ __forceinline__ void three_parts(float x, float y, uint32_t (&p)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    p[i] = pack_nearest(x, y);
+    x -= __uint_as_float(p[i] << 16);
+    y -= __uint_as_float(p[i] & 0xffff0000u);
+  }
+}
+__device__ __forceinline__ void bf16_mma(float (&d)[4], const uint32_t* a, const uint32_t* b) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-__device__ __forceinline__ void tf32_mma_from_zero(float (&d)[4], const uint32_t* a, const uint32_t* b) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+__device__ __forceinline__ void bf16_mma_from_zero(float (&d)[4], const uint32_t* a, const uint32_t* b) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.f));
 }
-// A 16 x 8 result of products of 16 x 8 (four values a lane, split here) and 8 x 8 values (in two parts): large and small
-// parts' products are summed apart.
+// A 16 x 8 result of products of 16 x 16 and 16 x 8 values in three parts: the first parts' products and the others' are summed
+// apart, the first parts' 16 at a time (the tensor cores' own sums round down) and then by 32-bit adds.  What is left out,
+// the second part times the third and the third times the third, is below 2^-25 of a product.
 struct TwoSums {
   float big[4], small[4];
   __device__ __forceinline__ void clear() {
@@ -131,19 +144,29 @@ struct TwoSums {
     for (int e = 0; e < 4; ++e) big[e] = small[e] = 0.f;
   }
   __device__ __forceinline__ float sum(int e) const { return big[e] + small[e]; }
-  __device__ __forceinline__ void add(const uint32_t* ah, const uint32_t* al, const uint32_t* bh, const uint32_t* bl) {
-    tf32_mma(small, al, bh);
-    tf32_mma(small, ah, bl);
-    float d[4];                                      // the tensor cores' own sums round down: eight products, then a 32-bit add
-    tf32_mma_from_zero(d, ah, bh);
+  __device__ __forceinline__ void add(const uint32_t (&a)[3][4], const uint32_t (&b)[3][2]) {
+    bf16_mma(small, a[2], b[0]);
+    bf16_mma(small, a[0], b[2]);
+    bf16_mma(small, a[1], b[1]);
+    bf16_mma(small, a[1], b[0]);
+    bf16_mma(small, a[0], b[1]);
+    float d[4];
+    bf16_mma_from_zero(d, a[0], b[0]);
 #pragma unroll
     for (int e = 0; e < 4; ++e) big[e] += d[e];
   }
 };
-__device__ __forceinline__ void tf32_parts4(const float (&x)[4], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+// A lane's 16 x 16 operand: x[2 i], x[2 i + 1] are neighbours along k of its register i.
+__device__ __forceinline__ void left_parts(const float2 (&x)[4], uint32_t (&a)[3][4]) {
 #pragma unroll
-  for (int e = 0; e < 4; ++e) tf32_parts(x[e], hi[e], lo[e]);
+  for (int i = 0; i < 4; ++i) {
+    uint32_t p[3];
+    three_parts(x[i].x, x[i].y, p);
+#pragma unroll
+    for (int n = 0; n < 3; ++n) a[n][i] = p[n];
+  }
 }
+__device__ __forceinline__ float2 pair_at(const float* p) { return *reinterpret_cast<const float2*>(p); }
 
 // ------------------------------------------------------------------------------------------- 1. scores
 // Within blocks of 16 tokens pair by pair with 32-bit multiply-adds, between blocks on the tensor cores.
@@ -154,7 +177,7 @@ __global__ void __launch_bounds__(SC_THREADS)
 channel_scores_kernel(const ChannelJob j) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) float sc[];
-  const int place = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, D = j.D, DP = D + 4;
+  const int place = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, D = j.D, DP = D + 8;
   float* Q = sc;                          // [RK][DP] q; later q times the decays since its block's begin
   float* K = Q + RK * DP;                 // k; later k times the decays up to its block's end
   float* A = K + RK * DP;                 // the decays; later k times the decays since its block's begin
@@ -274,27 +297,36 @@ channel_scores_kernel(const ChannelJob j) {
   for (int unit = warp; unit < (DELTA ? 12 : 6); unit += SC_THREADS / 32) {
     const int pair = unit % 6, fr = lane >> 2, fk = lane & 3;
     const int a = pair < 3 ? pair + 1 : (pair < 5 ? pair - 1 : 3), b = pair < 3 ? pair : (pair < 5 ? pair - 3 : 0);
-    const float* X = (unit < 6 ? Q : A) + (a * SUB + fr) * DP + fk;
-    const float* Y = K + (b * SUB + fr) * DP + fk;
+    const float* X = (unit < 6 ? Q : A) + (a * SUB + fr) * DP + 2 * fk;
+    const float* Y = K + (b * SUB + fr) * DP + 2 * fk;
     TwoSums sum[2];
     sum[0].clear();
     sum[1].clear();
-#pragma unroll 2
-    for (int c = 0; c < D; c += 8) {
-      float m0 = 1.f, m1 = 1.f;
-      for (int w = b + 1; w < a; ++w) {              // the whole blocks between
-        m0 *= B[w * D + c + fk];
-        m1 *= B[w * D + c + 4 + fk];
-      }
-      const float x[4] = {X[c], X[8 * DP + c], X[c + 4], X[8 * DP + c + 4]};
-      uint32_t xh[4], xl[4];
-      tf32_parts4(x, xh, xl);
+#pragma unroll 1
+    for (int c = 0; c < D; c += 16) {
+      float2 m[2] = {make_float2(1.f, 1.f), make_float2(1.f, 1.f)};
+      for (int w = b + 1; w < a; ++w)                // the whole blocks between
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float2 g = pair_at(B + w * D + c + 8 * i + 2 * fk);
+          m[i].x *= g.x;
+          m[i].y *= g.y;
+        }
+      const float2 x[4] = {pair_at(X + c), pair_at(X + 8 * DP + c), pair_at(X + c + 8), pair_at(X + 8 * DP + c + 8)};
+      uint32_t xp[3][4];
+      left_parts(x, xp);
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
-        uint32_t yh[2], yl[2];
-        tf32_parts(Y[8 * n * DP + c] * m0, yh[0], yl[0]);
-        tf32_parts(Y[8 * n * DP + c + 4] * m1, yh[1], yl[1]);
-        sum[n].add(xh, xl, yh, yl);
+        uint32_t yp[3][2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float2 y = pair_at(Y + 8 * n * DP + c + 8 * i);
+          uint32_t p[3];
+          three_parts(y.x * m[i].x, y.y * m[i].y, p);
+#pragma unroll
+          for (int t = 0; t < 3; ++t) yp[t][i] = p[t];
+        }
+        sum[n].add(xp, yp);
       }
     }
     float* to = unit < 6 ? po : ko;
@@ -320,7 +352,8 @@ channel_scores_kernel(const ChannelJob j) {
 }
 
 // ------------------------------------------------------------------------------------ 2. the triangular system
-// [W | U0] by forward substitution in blocks of 16 rows; a thread holds its column, so that nothing waits for another.
+// [W | U0] by forward substitution in blocks of 16 rows; a thread holds its column, so that nothing waits for another.  What is
+// taken off a row is summed by itself, so that its many small terms are not rounded to the row's own size one by one.
 constexpr int SO_COLS = 128;         // columns per block
 
 template <typename TV>
@@ -355,9 +388,12 @@ channel_solve_kernel(const ChannelJob j) {
   for (int r = 0; r < SUB; ++r) next[r] = right(r);
 #pragma unroll 1
   for (int b = 0; b < RK; b += SUB) {
-    float x[SUB];
+    float x[SUB], off[SUB];
 #pragma unroll
-    for (int r = 0; r < SUB; ++r) x[r] = bs[b + r] * next[r];
+    for (int r = 0; r < SUB; ++r) {
+      x[r] = bs[b + r] * next[r];
+      off[r] = 0.f;
+    }
     if (b + SUB < RK) {
 #pragma unroll
       for (int r = 0; r < SUB; ++r) next[r] = right(b + SUB + r);
@@ -368,17 +404,18 @@ channel_solve_kernel(const ChannelJob j) {
 #pragma unroll
       for (int r = 0; r < SUB; r += 4) {
         const float4 l = *reinterpret_cast<const float4*>(L + s * KK_PITCH + b + r);
-        x[r] = fmaf(-l.x, y, x[r]);
-        x[r + 1] = fmaf(-l.y, y, x[r + 1]);
-        x[r + 2] = fmaf(-l.z, y, x[r + 2]);
-        x[r + 3] = fmaf(-l.w, y, x[r + 3]);
+        off[r] = fmaf(l.x, y, off[r]);
+        off[r + 1] = fmaf(l.y, y, off[r + 1]);
+        off[r + 2] = fmaf(l.z, y, off[r + 2]);
+        off[r + 3] = fmaf(l.w, y, off[r + 3]);
       }
     }
 #pragma unroll
     for (int s = 0; s < SUB; ++s) {
+      x[s] -= off[s];
 #pragma unroll
       for (int r = 0; r < SUB; ++r)
-        if (r > s) x[r] = fmaf(-L[(b + s) * KK_PITCH + b + r], x[s], x[r]);
+        if (r > s) off[r] = fmaf(L[(b + s) * KK_PITCH + b + r], x[s], off[r]);
     }
 #pragma unroll
     for (int r = 0; r < SUB; ++r) {
@@ -392,9 +429,9 @@ channel_solve_kernel(const ChannelJob j) {
 // -------------------------------------------------------------------------------------------- 3. the walk
 // Two groups of eight warps share a chunk: the first moves the state on (W S, U, Kd^T U), the second reads out (Qd S, P U).
 // A warp has 16 tokens (or two times 16 key channels) x 8 value channels.  Bound by instruction issue and by the chain of a
-// chunk's two rounds of products and its barriers, 32 times for 2,048 tokens: the state and U are split into their tf32
-// parts once, where they are made.  16 value channels per block put 8 heads of 256 on 128 SMs.  With the conversion
-// instruction in the place of integer rounding the two forms took 209 and 286 us instead of 171 and 242.
+// chunk's two rounds of products and its two barriers, 32 times for 2,048 tokens: the state and U are split into their parts
+// once, where they are made.  16 value channels per block put 8 heads of 256 on 128 SMs.  Three bfloat16 parts take six
+// products of 16 x 8 x 16, as many as two tf32 parts' three of 16 x 8 x 8, and half the 32-bit adds (three tf32 parts: 249 and 332 us).
 constexpr int WK_THREADS = 512;
 
 __device__ __forceinline__ void wk_copy16(float* dst, const float* src) {
@@ -402,8 +439,8 @@ __device__ __forceinline__ void wk_copy16(float* dst, const float* src) {
 }
 
 size_t channel_walk_smem(int D, bool delta) {
-  const size_t rows = (size_t)RK * (D + 4), keys = (size_t)RK * (D + 8), p = (size_t)RK * KK_PITCH;
-  return (rows * (delta ? 2 : 1) + 2 * keys + 2 * p + 2 * D + (size_t)2 * (D + RK) * SP) * sizeof(float);
+  const size_t rows = (size_t)RK * (D + 8), keys = (size_t)RK * (D + 4), p = (size_t)RK * PP;
+  return (rows * (delta ? 2 : 1) + 2 * keys + 2 * p + 2 * D + (size_t)3 * (D + RK) / 2 * SP) * sizeof(float);
 }
 
 // The recurrence token by token with plain 32-bit multiply-adds, in the walk's own form (linear_attention.cu: read out the decayed
@@ -465,15 +502,15 @@ __global__ void __launch_bounds__(WK_THREADS)
 channel_walk_kernel(const __grid_constant__ ChannelJob j) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) float wk[];
-  const int D = j.D, QP = D + 4, KP = D + 8, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wr = warp & 3, wc = ((warp >> 2) & 1) * 8;
+  const int D = j.D, QP = D + 8, KP = D + 4, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wr = warp & 3, wc = ((warp >> 2) & 1) * 8;
   const bool moves = warp < 8;
   float* Q = wk;                                     // [RK][QP]
   float* W = Q + RK * QP;                            // delta rule only
   float* K = W + (DELTA ? RK * QP : 0);              // twice [RK][KP]
-  float* P = K + 2 * RK * KP;                        // twice [RK][KK_PITCH]
-  float* E = P + 2 * RK * KK_PITCH;                  // twice [D]: the chunk's decays
-  uint32_t* S = reinterpret_cast<uint32_t*>(E + 2 * D);       // the state's two parts, [D][SP] each
-  uint32_t* U = S + 2 * D * SP;                      // U's, [RK][SP] each
+  float* P = K + 2 * RK * KP;                        // twice [RK][PP]
+  float* E = P + 2 * RK * PP;                        // twice [D]: the chunk's decays
+  uint32_t* S = reinterpret_cast<uint32_t*>(E + 2 * D);       // the state's three parts, pairs of rows, [D / 2][SP] each
+  uint32_t* U = S + 3 * D / 2 * SP;                  // U's, [RK / 2][SP] each
   const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * RV;
   pdl_wait();
   const int tok0 = j.cu_q[seq], qlen = j.cu_q[seq + 1] - tok0;
@@ -497,7 +534,7 @@ channel_walk_kernel(const __grid_constant__ ChannelJob j) {
 #pragma unroll
     for (int e = tid; e < RK * RK / 4; e += WK_THREADS) {
       const int r = e / (RK / 4), s = (e - r * (RK / 4)) * 4;
-      if (s < (r & ~(SUB - 1)) + SUB) wk_copy16(P + buf * RK * KK_PITCH + r * KK_PITCH + s, p + r * RK + s);
+      if (s < (r & ~(SUB - 1)) + SUB) wk_copy16(P + buf * RK * PP + r * PP + s, p + r * RK + s);
     }
     if (tid * 4 < D) wk_copy16(E + buf * D + tid * 4, j.gend + at * D + tid * 4);
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -517,13 +554,15 @@ channel_walk_kernel(const __grid_constant__ ChannelJob j) {
   load_early(0);
   load_rows(0);
 
-  // x and y, in neighbouring columns, in two parts `gap` apart
-  auto put_parts = [&](uint32_t* to, int gap, float x, float y) {
-    uint32_t xh, xl, yh, yl;
-    tf32_parts(x, xh, xl);
-    tf32_parts(y, yh, yl);
-    *reinterpret_cast<uint2*>(to) = make_uint2(xh, yh);
-    *reinterpret_cast<uint2*>(to + gap) = make_uint2(xl, yl);
+  // A product's results x and y, in columns fc and fc + 1 of row `row`, in three parts `gap` apart, by the whole warp: the lane of
+  // the even row of two stores both rows' column fc, the other one their column fc + 1.
+  const int odd = fr & 1;
+  auto put_parts = [&](uint32_t* to, int gap, int row, float x, float y) {
+    const float other = __shfl_xor_sync(0xffffffffu, odd ? x : y, 4);
+    uint32_t p[3];
+    three_parts(odd ? other : x, odd ? y : other, p);
+#pragma unroll
+    for (int n = 0; n < 3; ++n) to[n * gap + (row >> 1) * SP + fc + odd] = p[n];
   };
   // the state: key channels (wr + 4 m) 16 .., in the first group's registers as a product's results lie
   float st[2][4] = {};
@@ -532,8 +571,8 @@ channel_walk_kernel(const __grid_constant__ ChannelJob j) {
     for (int m = 0; m < 2; ++m) {
       const int row = (wr + 4 * m) * 16 + fr;
       if (!moves || (wr + 4 * m) * 16 >= D) continue;
-      put_parts(S + row * SP + fc, D * SP, st[m][0], st[m][1]);
-      put_parts(S + (row + 8) * SP + fc, D * SP, st[m][2], st[m][3]);
+      put_parts(S, D / 2 * SP, row, st[m][0], st[m][1]);
+      put_parts(S, D / 2 * SP, row + 8, st[m][2], st[m][3]);
     }
   };
   auto each = [&](auto f) {
@@ -550,15 +589,31 @@ channel_walk_kernel(const __grid_constant__ ChannelJob j) {
   each([](float& x, float* at) { x = *at; });
   share_state();
 
-  // 16 x 8 values at `a` (pitch `row` between its rows, `col` between its columns) times 8 rows of two parts
-  auto step = [&](TwoSums& sum, const float* a, int row, int col, const uint32_t* b, int gap) {
-    const float x[4] = {a[0], a[8 * row], a[4 * col], a[8 * row + 4 * col]};
-    uint32_t ah[4], al[4];
-    tf32_parts4(x, ah, al);
-    const uint32_t bh[2] = {b[0], b[4 * SP]}, bl[2] = {b[gap], b[gap + 4 * SP]};
-    sum.add(ah, al, bh, bl);
+  // 16 x 16 values times 16 rows of three parts
+  auto step = [&](TwoSums& sum, const float2 (&x)[4], const uint32_t* b, int gap) {
+    uint32_t ap[3][4], bp[3][2];
+    left_parts(x, ap);
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+      bp[n][0] = b[n * gap];
+      bp[n][1] = b[n * gap + 4 * SP];
+    }
+    sum.add(ap, bp);
   };
-  const int frag = fk * SP + wc + fr;                // this lane's place in 8 rows of S or U
+  auto along_row = [&](TwoSums& sum, const float* a, int pitch, const uint32_t* b, int gap) {
+    const float2 x[4] = {pair_at(a), pair_at(a + 8 * pitch), pair_at(a + 8), pair_at(a + 8 * pitch + 8)};
+    step(sum, x, b, gap);
+  };
+  auto along_column = [&](TwoSums& sum, const float* a, int pitch, const uint32_t* b, int gap) {
+    float2 x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float* p = a + (i >> 1) * 8 * pitch + (i & 1) * 8;
+      x[i] = make_float2(p[0], p[pitch]);
+    }
+    step(sum, x, b, gap);
+  };
+  const int frag = fk * SP + wc + fr;                // this lane's place in 8 pairs of rows of S or U
 
   TwoSums sum;
   bool finite = true;                                // the outputs, and at the end the state: neither forgets a value that is no number
@@ -584,22 +639,22 @@ channel_walk_kernel(const __grid_constant__ ChannelJob j) {
     if (i + 1 < chunks) load_early(i + 1);            // the chunk before is done with these buffers
     sum.clear();
     if (DELTA || !moves) {
-      const float* A = (moves ? W : Q) + (wr * 16 + fr) * QP + fk;
-#pragma unroll 4
-      for (int c = 0; c < D; c += 8) step(sum, A + c, QP, 1, S + c * SP + frag, D * SP);
+      const float* A = (moves ? W : Q) + (wr * 16 + fr) * QP + 2 * fk;
+#pragma unroll 2
+      for (int c = 0; c < D; c += 16) along_row(sum, A + c, QP, S + c / 2 * SP + frag, D / 2 * SP);
     }
     if (moves) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) u[e] = DELTA ? u[e] - sum.sum(e) : u[e];
-      put_parts(U + (wr * 16 + fr) * SP + fc, RK * SP, u[0], u[1]);
-      put_parts(U + (wr * 16 + fr + 8) * SP + fc, RK * SP, u[2], u[3]);
+      put_parts(U, RK / 2 * SP, wr * 16 + fr, u[0], u[1]);
+      put_parts(U, RK / 2 * SP, wr * 16 + fr + 8, u[2], u[3]);
     }
     __syncthreads();                                  // U is there; nobody reads Q, W and the state any more
     if (i + 1 < chunks) load_rows(i + 1);
     if (!moves) {
-      const float* A = P + buf * RK * KK_PITCH + (wr * 16 + fr) * KK_PITCH + fk;
-#pragma unroll 2
-      for (int c = 0; c < (wr + 1) * 16; c += 8) step(sum, A + c, KK_PITCH, 1, U + c * SP + frag, RK * SP);
+      const float* A = P + buf * RK * PP + (wr * 16 + fr) * PP + 2 * fk;
+#pragma unroll 1
+      for (int c = 0; c < (wr + 1) * 16; c += 16) along_row(sum, A + c, PP, U + c / 2 * SP + frag, RK / 2 * SP);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int t = wr * 16 + fr + (e >> 1) * 8, col = v0 + fc + (e & 1);
@@ -610,14 +665,14 @@ channel_walk_kernel(const __grid_constant__ ChannelJob j) {
         }
       }
     } else {
-      const float* Kb = K + buf * RK * KP + fk * KP + fr;
+      const float* Kb = K + buf * RK * KP + 2 * fk * KP + fr;
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
         const int c0 = (wr + 4 * m) * 16;
         if (c0 >= D) continue;
         sum.clear();
-#pragma unroll 4
-        for (int s = 0; s < RK; s += 8) step(sum, Kb + s * KP + c0, 1, KP, U + s * SP + frag, RK * SP);
+#pragma unroll 2
+        for (int s = 0; s < RK; s += 16) along_column(sum, Kb + s * KP + c0, KP, U + s / 2 * SP + frag, RK / 2 * SP);
         const float g[2] = {E[buf * D + c0 + fr], E[buf * D + c0 + fr + 8]};
 #pragma unroll
         for (int e = 0; e < 4; ++e) st[m][e] = fmaf(g[e >> 1], st[m][e], sum.sum(e));
@@ -692,7 +747,7 @@ extern "C" int zi_channel_recurrence(float* out, int ldo, const void* q, int ldq
     zi_launch(kern, grid, dim3(threads), smem, stream, j);
     return zi_check_launch(what);
   };
-  const size_t score_smem = ((size_t)3 * RK * (D + 4) + 3 * SUBS * D) * sizeof(float);
+  const size_t score_smem = ((size_t)3 * RK * (D + 8) + 3 * SUBS * D) * sizeof(float);
   const size_t solve_smem = ((size_t)RK * KK_PITCH + RK + (size_t)RK * SO_COLS) * sizeof(float);
   int rc = 0;
   ZI_DISPATCH_DTYPE(qk_dtype, TQ, {

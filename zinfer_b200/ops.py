@@ -1936,7 +1936,7 @@ def _channel_chunks_pay(longest: int, tokens: int, delta: bool) -> bool:
 def channel_decay_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, beta: Optional[torch.Tensor],
                              q_scale: float, state: torch.Tensor, heads: int, key_heads: int, dim: int, vdim: int, step, fast: bool) -> torch.Tensor:
     """The recurrence with one decay per key channel, between 0 and 1 (see :func:`linear_recurrence`; with ``beta`` the delta
-    rule): token by token, or, where ``fast`` allows the tensor cores' products (each operand in two tf32 parts) and a portion is
+    rule): token by token, or, where ``fast`` allows the tensor cores' products (each operand in three bfloat16 parts, all its bits) and a portion is
     long, in chunks of 64 tokens, single tokens of the same step token by token.  Returns float32 [T, heads * vdim]."""
     T = q.shape[0]
     L = lib()
