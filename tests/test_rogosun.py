@@ -629,6 +629,19 @@ def test_recurrence_in_chunks_is_no_further_from_64_bits_than_the_walk(delta, q_
     assert all(c <= w for c, w in zip(errors[True], errors[False])), errors
 
 
+def test_single_tokens_take_no_room_of_the_chunks():
+    """The workspace of a step: the chunks of its longer portions, whatever decodes beside them."""
+    from zinfer_b200 import ops
+
+    size = lambda q_lens: ops.lib().zi_channel_recurrence_workspace_floats(sum(q_lens), len(q_lens), q_lens.count(1), 8, 128, 256, 1)
+    chunk = 8 * (64 * (3 * 128 + 2 * 64 + 256) + 128)              # q, k, W; both scores; U; the chunk's decays
+    for q_lens in ([160], [65, 2, 64], [300, 63]):
+        needed = sum(-(-n // 64) for n in q_lens) * chunk
+        assert needed <= size(q_lens) <= needed + len(q_lens) * chunk
+        assert size(q_lens + [1] * 256) == size(q_lens)
+    assert size([1] * 8) == 0
+
+
 @gpu
 @pytest.mark.parametrize("delta", [False, True])
 @pytest.mark.parametrize("what", ["q", "k", "v", "decay", "beta", "state"])
