@@ -629,6 +629,29 @@ def test_recurrence_in_chunks_is_no_further_from_64_bits_than_the_walk(delta, q_
     assert all(c <= w for c, w in zip(errors[True], errors[False])), errors
 
 
+# (delta rule, key channels, value channels, heads, tokens per request, us of the walk, us in chunks), measured on one B200
+MEASURED_RECURRENCES = [
+    (False, 128, 256, 8, [32], 16, 26), (False, 128, 256, 8, [96], 40, 34), (False, 128, 256, 8, [2048], 758, 182),
+    (False, 128, 256, 8, [32] * 8, 60, 70), (False, 128, 256, 8, [64] * 8, 107, 74), (False, 128, 256, 8, [48] + [1] * 200, 417, 490),
+    (False, 128, 256, 8, [512] + [1] * 24, 246, 125), (True, 128, 256, 8, [96], 45, 60), (True, 128, 256, 8, [128], 58, 67),
+    (True, 128, 256, 8, [192], 84, 73), (True, 128, 256, 8, [48] * 9, 95, 112), (True, 128, 256, 8, [64] * 8, 120, 107),
+    (True, 128, 256, 8, [100] + [1] * 16, 86, 110), (True, 128, 256, 8, [160] + [1] * 64, 214, 228), (True, 128, 256, 8, [512] + [1] * 24, 271, 165),
+    (False, 16, 8, 2, [32] * 8, 13, 18), (False, 16, 8, 2, [256], 83, 25), (True, 16, 8, 2, [64] * 32, 25, 51), (True, 16, 8, 2, [256], 89, 46),
+    (False, 64, 64, 4, [64] * 32, 26, 44), (False, 64, 64, 4, [256], 92, 32), (True, 64, 64, 4, [48] * 9, 22, 52), (True, 64, 64, 4, [100] * 10, 42, 57),
+    (True, 64, 64, 4, [256], 98, 53), (False, 128, 128, 16, [64] * 32, 376, 281), (True, 128, 128, 16, [64], 32, 61),
+]
+
+
+@pytest.mark.parametrize("delta,D,V,H,q_lens,walk,chunks", MEASURED_RECURRENCES)
+def test_recurrences_run_in_the_form_that_measured_faster(delta, D, V, H, q_lens, walk, chunks):
+    """The choice between the walk and the chunks, by heads, channels and the step's requests: single tokens beside a portion
+    count for neither."""
+    from zinfer_b200 import ops
+
+    step = SimpleNamespace(n_seqs=len(q_lens), n_dec=q_lens.count(1), max_q_len=max(q_lens), q_lens=q_lens)
+    assert ops._channel_chunks_pay(step, sum(q_lens), H, D, V, delta) == (chunks < walk)
+
+
 def test_single_tokens_take_no_room_of_the_chunks():
     """The workspace of a step: the chunks of its longer portions, whatever decodes beside them."""
     from zinfer_b200 import ops

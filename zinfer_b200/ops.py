@@ -1925,12 +1925,25 @@ RECURRENCE_CHUNKS = os.environ.get("ZINFER_B200_RECURRENCE_CHUNKS", "1") not in 
 RECURRENCE_CHUNK_MIN = 96     # from this many tokens in a request's portion the chunked form pays
 
 
-def _channel_chunks_pay(longest: int, tokens: int, delta: bool) -> bool:
-    """Whether a step's portions with one decay per key channel run in chunks: the walk takes 0.37 us a token of the longest portion
-    until its blocks fill the GPU, the chunks 40 us (delta rule 60) and 0.06 (0.09) us a token.  Measured at 8 heads of 128 x 256, us
-    (walk, chunks): plain 1 x 96 39.7, 40.3; 1 x 256 98, 45; 8 x 64 107, 66; 4 x 32 31, 43; delta rule 1 x 128 57, 68; 1 x 256 109, 74;
-    8 x 64 120, 102; 4 x 32 35, 70."""
-    return longest >= (160 if delta else 112) or (longest >= 48 and tokens >= 400)
+def _channel_chunks_pay(step, tokens: int, heads: int, dim: int, vdim: int, delta: bool) -> bool:
+    """Whether a step's portions with one decay per key channel run in chunks, by what either form takes, us on one B200.  The
+    walk: 0.365 a token of the longest portion (delta rule 0.4), or, once its blocks fill the GPU, 0.19 (0.21) a token of all and 1.9 a
+    request with one token, for 8 heads of 128 x 256 (``work`` is a step's share of that).  The chunks: 22 (45), 4.4 a chunk of the
+    longest portion or 6.6 (7.6) a chunk of all, and the requests with one token behind them.  They have to promise 3 us.  Measured
+    (walk, chunks), 8 heads of 128 x 256, plain: 1 x 64 28, 30; 1 x 96 40, 34; 8 x 32 60, 70; 8 x 64 107, 74; 48 beside 200 single
+    tokens 417, 490; delta rule: 1 x 128 58, 67; 1 x 192 84, 73; 9 x 48 95, 112; 8 x 64 120, 107; 160 beside 64 single tokens 214, 228;
+    4 heads of 64 x 64: 32 x 64 plain 26, 44, delta rule 28, 75, 1 x 256 92, 32 and 98, 53."""
+    singles, longest = step.n_dec, step.max_q_len
+    multi = step.n_seqs - singles
+    if multi == 0 or longest < 32:
+        return False
+    lens = getattr(step, "q_lens", None)
+    chunks = sum((n + 63) // 64 for n in lens if n > 1) if lens else (tokens - singles) / 64 + multi / 2
+    work = heads * dim * vdim / (8 * 128 * 256)
+    alone = 1.9 * singles * work
+    walk = 6 + max((0.4 if delta else 0.365) * longest, (0.21 if delta else 0.19) * (tokens - singles) * work + alone)
+    in_chunks = (45 if delta else 22) + max(4.4 * ((longest + 63) // 64), (7.6 if delta else 6.6) * chunks * work) + alone + (2 if singles else 0)
+    return in_chunks + 3 < walk
 
 
 def channel_decay_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, beta: Optional[torch.Tensor],
@@ -1941,7 +1954,7 @@ def channel_decay_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
     T = q.shape[0]
     L = lib()
     delta = beta is not None
-    if not (fast and RECURRENCE_CHUNKS and _channel_chunks_pay(step.max_q_len, T, delta) and L.zi_channel_recurrence_supported(dim, vdim, heads, key_heads)):
+    if not (fast and RECURRENCE_CHUNKS and _channel_chunks_pay(step, T, heads, dim, vdim, delta) and L.zi_channel_recurrence_supported(dim, vdim, heads, key_heads)):
         return linear_recurrence(q, k, v, decay, beta, q_scale, state, heads, key_heads, dim, vdim, step)
     st, stride = _slot_view(state, "channel_decay_recurrence")
     _need(st[0].numel() == heads * dim * vdim, "channel_decay_recurrence: state [slots, heads, dim, vdim]")
