@@ -100,6 +100,23 @@ def test_the_switch_of_cta_pairs_gives_back_what_it_found(env, first):
     assert r.returncode == 0, r.stderr[-2000:]
 
 
+@pytest.mark.parametrize("M,N,K,splits", [
+    # on pairs with so many splits, us on one B200 (single -> pair): 266 against 333, 127 against 144, 61 against 70 (with the
+    # reader of the sums; 65 whole), 64 against 71, 42 against 45 (with the reader)
+    (2048, 24576, 4096, 1), (1536, 4096, 12288, 1), (536, 4096, 12288, 3), (675, 4096, 12288, 1), (300, 4096, 12288, 2),
+    # left to the single-CTA kernel (single, best of the pairs): 12.9 and 16.5 with the reader, 13.0 and 16.4, 11.9 and 13.2, 5.1 and
+    # 5.7, 5.2 and 5.7, 6.2 and 7.0, 17.3 and 18.4
+    (129, 4096, 4096, 0), (129, 2048, 8448, 0), (1300, 3072, 1024, 0), (512, 256, 256, 0), (256, 256, 256, 0), (257, 512, 512, 0), (675, 5120, 2048, 0)])
+def test_pairs_are_planned_where_they_measured_faster(M, N, K, splits):
+    if shutil.which("nvcc") is None:
+        pytest.skip("no nvcc to build the kernel library with")
+    from zinfer_b200 import ops
+
+    plan = (ctypes.c_int * 4)()
+    ops.lib().zi_gemm_tcgen05_plan_for(M, N, K, 148, 74, plan)
+    assert plan[3] == (splits > 0) and (not splits or plan[2] == splits)
+
+
 def test_splits_never_leave_a_split_without_k_blocks(plan):
     for M in (1, 8, 64, 65, 128, 300):
         for N, K in [(128, 64), (256, 512), (1000, 264), (4096, 4096), (5120, 17408), (151936, 4096)]:

@@ -825,11 +825,15 @@ int pair_mode() {
 }
 
 // The kernel for CTA pairs, or not, and its K splits.  Time in whole rounds of tiles: a k-block of a single CTA's 128 x 256
-// (or 128 x 128) tile takes 0.37 (0.31) us, of a pair's 256 x 256 tile 0.335 us (measured on full rounds of real weights; with
-// operands from L2 0.32, 0.31 and 0.29).  Splitting K writes the sums as floats and reads them back, about 6 TB/s in L2,
-// and 3 us more; it has to promise 8 us, for the model is no better than that.  Measured, us (single -> pair): 2048 x 24576 x
-// 4096 282 -> 265, 2048 x 4096 x 12288 156 -> 144, 1024 x 4096 x 12288 80 -> 74, 512 x 24576 x 4096 89 -> 80.  `slots`: pairs
-// resident at once (resident_pairs).
+// (or 128 x 128) tile takes 0.37 (0.25) us, of a pair's 256 x 256 tile 0.32, and a pair's launch and last drain 3 us more than
+// a single's.  Splitting K writes the sums as floats and reads them back, about 6 TB/s in L2, and 3 us more; it has to promise
+// 8 us, for a caller may want the sums added up.  The figures are those that choose best over 332 products of 129 to 3,000 tokens,
+// N of 256 to 24,576 and K of 256 to 12,288, timed in graphs with weights from memory: with the reader of the sums counted, 4 are
+// chosen more than 2 % slower than the single-CTA kernel (4 % at most: 129 x 24576 x 4096) and the mean is 0.8 % off the
+// best plan of either kernel.  Measured, us (single -> pair): 2048 x 24576 x 4096 333 -> 266, 1536 x 4096 x 12288 144 -> 127,
+// 536 x 4096 x 12288 with its sums' reader 70 -> 61 (three splits; whole 65), 675 x 4096 x 12288 71 -> 64; and where the single
+// kernel stays: 129 x 4096 x 4096 12.9 against 16.5 on pairs, 1300 x 3072 x 1024 11.9 against 13.2, 512 x 256 x 256 5.1 against 5.7.
+// `slots`: pairs resident at once (resident_pairs).
 bool plan_pair(int M, int N, int K, int sm_count, int slots, int* plan) {
   const int mode = pair_mode();
   if (mode == PAIR_NEVER || plan[0] || N < PAIR_TILE || slots <= 0) return false;
@@ -846,12 +850,12 @@ bool plan_pair(int M, int N, int K, int sm_count, int slots, int* plan) {
   };
   const long long singles = (long long)((M + TILE_A - 1) / TILE_A) * ((N + plan[1] - 1) / plan[1]);
   const long long pairs = (long long)((M + PAIR_TILE - 1) / PAIR_TILE) * ((N + PAIR_TILE - 1) / PAIR_TILE);
-  const double single = time(singles, sms, plan[2], plan[1] >= 256 ? 0.37 : 0.31);
-  const double whole = time(pairs, slots, 1, 0.335);
+  const double single = time(singles, sms, plan[2], plan[1] >= 256 ? 0.37 : 0.25);
+  const double whole = time(pairs, slots, 1, 0.32) + 3.0;
   double best = whole;
   int splits = 1;
-  for (int s = 2; s <= 8 && k_blocks / s >= 8; ++s) {
-    const double t = time(pairs, slots, s, 0.335);
+  for (int s = 2; s <= 8 && k_blocks / s >= 8 && pairs * s <= 2 * slots; ++s) {      // (measured up to two rounds)
+    const double t = time(pairs, slots, s, 0.32) + 3.0;
     if (t < best && t < whole - 8.0) {
       best = t;
       splits = s;
