@@ -226,9 +226,12 @@ namespace {
 // Measured, us on one B200 (rows x columns x K; the plain kernel -> the tile taken; every output's bits are the same):
 //   1 x 1024 x 1024  106 -> 5.4      12 x 1024 x 1024  106 -> 8.5     12 x 6144 x 1024  126 -> 14.2   12 x 1024 x 3072  311 -> 21.7
 //   30 x 1024 x 1024  11.4           100 x 1024 x 1024  26            512 x 1024 x 1024  101 -> 41    512 x 6144 x 1024  336 -> 187
-// and with the tile next to the line: 12 x 6144 x 1024 in tiles of 8 columns 18.3, 12 x 32768 x 1024 in tiles of 16 69.9
-// against 63.1 of 32; 100 x 1024 x 1024 in 32 x 32 tiles 38; 512 x 1024 x 3072 in 64 x 64 tiles 342 against 120 of 32 x 32,
-// 512 x 6144 x 1024 in 32 x 32 tiles 222.
+// The lines lie where a tile's blocks no longer are all resident at once (three an SM of the 16 x 8 and 16 x 16 tiles, four of
+// the 64 x 64): 12 x 3072 x 1024 in tiles of 8 | 16 | 32 columns 9.5 | 13.9 | 21, x 3600 15.3 | 14.0 | 20.9, x 7104 19.2 | 15.2 | 16.9,
+// x 7500 24.6 | 28.2 | 22.5, x 11840 36.0 | 29.2 | 23.3; 3 x 4096 x 1024 in tiles of 8 | 32 7.1 | 9.8, x 6144 12.2 | 9.7; 24 x 2048 x
+// 1024 in tiles of 8 | 16 11.6 | 21.8, x 3072 22.5 | 22.4; 100 x 1024 x 1024 in 32 x 32 tiles 38.  In 32 x 32 | 64 x 64 tiles:
+// 512 x 2816 x 1024 106 | 118, 512 x 3072 x 1024 120 | 118, 512 x 4608 x 1024 161 | 118, 300 x 6144 x 1024 144 | 118, 512 x 5632 x 1024
+// 200 | 187, 512 x 6144 x 1024 222 | 187, 512 x 1024 x 3072 120 | 342.
 constexpr int SMS = 148;
 template <typename TO>
 int launch_f32(void* out, const float* x, const float* w, int M, int N, int K, int ldx, int ldw, int ldo, int early,
@@ -243,8 +246,8 @@ int launch_f32(void* out, const float* x, const float* w, int M, int N, int K, i
       ZI_FEW(4, 32, 2, 1, 128, 4, 7);
     }
     if (M <= 16) {
-      if (N <= 16 * SMS) ZI_FEW(16, 8, 2, 1, 256, 3, 3);
-      if (N <= 80 * SMS) ZI_FEW(16, 16, 2, 2, 128, 4, 3);
+      if (N <= 24 * SMS) ZI_FEW(16, 8, 2, 1, 256, 3, 3);
+      if (N <= 48 * SMS) ZI_FEW(16, 16, 2, 2, 128, 4, 3);
       ZI_FEW(16, 32, 2, 2, 128, 3, 3);
     }
     if (M <= 32) {
@@ -254,7 +257,8 @@ int launch_f32(void* out, const float* x, const float* w, int M, int N, int K, i
     ZI_FEW(32, 16, 4, 2, 128, 3, 3);
 #undef ZI_FEW
   }
-  if (blocks64 >= 5 * SMS) return launch_f32_tile<F32Tile<64, 64, 8, 8, 32, 3, 1>, TO>(out, x, w, M, N, K, ldx, ldw, ldo, early, stream);
+  // 64 x 64 tiles: one round of four an SM takes as long as 32 x 32 tiles of 10 an SM; past it they pay again from 4.6 an SM on
+  if (blocks64 > 4 * SMS ? 10 * blocks64 >= 46 * SMS : blocks32 > 10 * SMS) return launch_f32_tile<F32Tile<64, 64, 8, 8, 32, 3, 1>, TO>(out, x, w, M, N, K, ldx, ldw, ldo, early, stream);
   return launch_f32_tile<F32Tile<32, 32, 4, 4, 64, 3, 2>, TO>(out, x, w, M, N, K, ldx, ldw, ldo, early, stream);
 }
 }  // namespace
