@@ -749,3 +749,23 @@ def test_decays_of_a_low_rank_pair(T, N, rank, dim):
         got = ops.low_rank_decay(x, w, bias, a_log if a else None, 16.0, dim)
         # z of size up to 4 sqrt(rank), its roundings and those of exp, log1p: 2^-18 of the exponent's slope, which is at most |z| e^a
         assert torch.allclose(got.double(), exact, rtol=2e-5, atol=1e-6)
+
+
+def test_decays_of_a_low_rank_pair_want_whole_heads(monkeypatch):
+    """Channels that are no whole number of heads were refused with the product and the decay's kernel and are with one kernel
+    (whose last channels would read beyond ``a_log``)."""
+    from zinfer_b200 import ops
+
+    class OnGpu(torch.Tensor):
+        is_cuda = True
+
+    launched = []
+    monkeypatch.setattr(ops, "lib", lambda: SimpleNamespace(zi_low_rank_decay=lambda *a: launched.append(a) or 0))
+    monkeypatch.setattr(ops, "_ptr", lambda t: None)
+    monkeypatch.setattr(ops, "_stream", lambda: None)
+    x, w = torch.zeros(2, 4, dtype=torch.bfloat16).as_subclass(OnGpu), torch.zeros(20, 4, dtype=torch.bfloat16)
+    with pytest.raises(ops.KernelError):
+        ops.low_rank_decay(x, w, torch.zeros(20), torch.zeros(2), 1.0, 8)
+    assert not launched
+    ops.low_rank_decay(x, w[:16], torch.zeros(16), torch.zeros(2), 1.0, 8)
+    assert len(launched) == 1

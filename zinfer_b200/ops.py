@@ -1856,6 +1856,7 @@ def low_rank_decay(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor
         z = linear(x, w, out_dtype=torch.float32)
         return decay_exp_softplus_(z, bias, a_log, head_dim) if a_log is not None else decay_sigmoid_root_(z, bias, tau)
     _need(w.shape[1] == rank, "low_rank_decay: the two matrices share their rank")
+    _need(a_log is None or a_log.numel() * head_dim == N, "low_rank_decay: a_log float32 [heads]")
     for v, n in ((bias, N), (a_log, N // head_dim)):
         _need(v is None or (v.dtype == torch.float32 and v.numel() == n and v.is_contiguous()), "low_rank_decay: bias and a_log are float32")
     out = torch.empty((T, N), dtype=torch.float32, device=x.device)
