@@ -1,13 +1,13 @@
 // Long portions of the recurrences with one decay per key channel and token (linear_attention.cu has the form that walks
 // the tokens one by one), in chunks of 64 tokens whose work is matrix products:
 //
-//     S <- diag(g_t) S ;  u_t = v_t  or  beta_t v_t  or  beta_t (v_t - S^T k_t) (delta rule) ;  S <- S + k_t u_t^T ;  o_t = S^T q_t
+//     S <- diag(g_t) S ;  u_t = v_t  or  beta_t (v_t - S^T k_t) (delta rule) ;  S <- S + k_t u_t^T ;  o_t = S^T q_t
 //
 // With G(a, b] the product of the decays of tokens a + 1 .. b (a vector over the key channels) inside a chunk that begins
 // from S0, and * the product by channels:
 //
 //     P_ts = sum_i q_ti k_si G(s, t]_i  for s <= t,    L_ts = beta_t sum_i k_ti k_si G(s, t]_i  for s < t,
-//     (I + L) [W | U0] = diag(beta) [k_t * G(0, t] | V] ,   U = U0 - W S0   (without the delta rule U = V or diag(beta) V),
+//     (I + L) [W | U0] = diag(beta) [k_t * G(0, t] | V] ,   U = U0 - W S0   (without the delta rule U = V),
 //     O = (q_t * G(0, t]) S0 + P U ,   S1 = diag(G(0, 64]) S0 + (k_s * G(s, 64])^T U
 //
 // (the chunked form of "Gated Linear Attention Transformers with Hardware-Efficient Training", Yang et al., 2023, and of
@@ -486,8 +486,7 @@ __device__ __noinline__ void walk_tokens(const ChannelJob& j, float* state, floa
       for (int w = 0; w < WARPS; ++w) sum[n] += red[(n * WARPS + w) * RV + c];
     }
     float u = on ? to_f32(static_cast<const TV*>(j.v)[(size_t)(tok0 + t) * j.ldv + (size_t)h * j.V + col]) : 0.f;
-    if (DELTA) u -= sum[0];
-    if (j.beta) u *= j.beta[(size_t)(tok0 + t) * j.ldb + h];
+    if (DELTA) u = j.beta[(size_t)(tok0 + t) * j.ldb + h] * (u - sum[0]);
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) st[r] = fmaf(kt[r], u, st[r]);
     if (on && i0 == 0) j.out[(size_t)(tok0 + t) * j.ldo + (size_t)h * j.V + col] = fmaf(u, sum[2], sum[1]);
@@ -626,12 +625,8 @@ channel_walk_kernel(const __grid_constant__ ChannelJob j) {
       const int t = wr * 16 + fr + (e >> 1) * 8, col = v0 + fc + (e & 1);
       u[e] = 0.f;
       if (moves && t < n && col < j.V) {
-        if (DELTA) {
-          u[e] = j.u0[(((size_t)(place0 + i) * j.H + h) * RK + t) * j.V + col];
-        } else {
-          u[e] = to_f32(static_cast<const TV*>(j.v)[(size_t)(first + t) * j.ldv + (size_t)h * j.V + col]);
-          if (j.beta) u[e] *= j.beta[(size_t)(first + t) * j.ldb + h];
-        }
+        u[e] = DELTA ? j.u0[(((size_t)(place0 + i) * j.H + h) * RK + t) * j.V + col]
+                     : to_f32(static_cast<const TV*>(j.v)[(size_t)(first + t) * j.ldv + (size_t)h * j.V + col]);
       }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -714,7 +709,7 @@ extern "C" long long zi_channel_recurrence_workspace_floats(int T, int n_seqs, i
 }
 
 // The portions of two tokens and more of a step; the n_single requests that bring one token are left alone.  decay: float32 [T][H * D],
-// between 0 and 1; beta: step sizes [T][H] or null (then without the delta rule); q and k of one type, v of its own;
+// between 0 and 1; beta: step sizes [T][H], with the delta rule and only there; q and k of one type, v of its own;
 // workspace: zi_channel_recurrence_workspace_floats, 16-byte aligned.
 extern "C" int zi_channel_recurrence(float* out, int ldo, const void* q, int ldq, const void* k, int ldk, int qk_dtype, const void* v,
                                      int ldv, int v_dtype, const float* decay, int ldg, const float* beta, int ldb, float q_scale,
@@ -725,8 +720,8 @@ extern "C" int zi_channel_recurrence(float* out, int ldo, const void* q, int ldq
   const int places = channel_places(T, n_seqs, n_single);
   if (places == 0) return 0;
   if (!zi_channel_recurrence_supported(D, V, H, G)) return zi_refuse("channel_recurrence: %d heads (%d of keys) of %d x %d", H, G, D, V);
-  if (!workspace || ((uintptr_t)workspace & 15) || !decay || (delta && !beta))
-    return zi_refuse("channel_recurrence: needs decays, with the delta rule steps, and an aligned workspace");
+  if (!workspace || ((uintptr_t)workspace & 15) || !decay || (delta != 0) != (beta != nullptr))
+    return zi_refuse("channel_recurrence: needs decays, with the delta rule (and only there) steps, and an aligned workspace");
   const ChannelPlan p = channel_plan(places, H, D, V, delta);
   ChannelJob j = {};
   j.q = q; j.k = k; j.v = v; j.decay = decay; j.beta = beta;
