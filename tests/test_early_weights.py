@@ -45,16 +45,25 @@ def test_32_bit_products_read_weights_early_only_when_told(recorder):
     assert early(recorder, "zi_gemm_simt") == 0
 
 
-def test_norms_of_updates_and_decays_read_nothing_before_their_wait():
-    """In the kernels themselves: the wait for earlier kernels stands before the first read of an operand."""
+def test_norms_of_updates_read_nothing_before_their_wait():
+    """In the kernel itself: the wait for earlier kernels stands before the first read of an operand."""
     import os
     import re
 
-    for f, kernel in (("elementwise.cu", "norm_residual_few_kernel"), ("linear_attention.cu", "low_rank_decay_kernel")):
-        with open(os.path.join(os.path.dirname(ops.__file__), "csrc", f)) as fh:
-            body = fh.read().split(kernel + "(", 1)[1].split("{", 1)[1]
-        before = body[:body.index("pdl_wait();")]
-        assert not re.search(r"\b(w|bias|a_log|x|h|a|ap|b|bp)\s*\[|load\(", before), kernel
+    with open(os.path.join(os.path.dirname(ops.__file__), "csrc", "elementwise.cu")) as fh:
+        body = fh.read().split("norm_residual_few_kernel(", 1)[1].split("{", 1)[1]
+    before = body[:body.index("pdl_wait();")]
+    assert not re.search(r"\b(w|bias|a_log|x|h|a|ap|b|bp)\s*\[|load\(", before)
+
+
+def test_decays_read_weights_early_only_when_told(recorder):
+    class OnGpu(torch.Tensor):
+        is_cuda = True
+
+    x, pair = torch.zeros(2, 4, dtype=torch.bfloat16).as_subclass(OnGpu), torch.zeros(8, 4, dtype=torch.bfloat16)
+    for said, want in (({}, 0), ({"fresh_weights": True}, 0), ({"fresh_weights": False}, 1)):
+        ops.low_rank_decay(x, pair, torch.zeros(8), None, 16.0, 4, **said)
+        assert early(recorder, "zi_low_rank_decay") == want
 
 
 def test_models_say_that_their_weights_are_weights():

@@ -227,7 +227,7 @@ int zi_short_conv_carry(float* tail, long long slot_stride, const void* x, int l
 int zi_decay(float* z, long long rows, int N, int D, const float* bias, const float* a_log, float inv_tau, int mode,
              cudaStream_t stream);
 int zi_low_rank_decay(float* out, const void* x, int ldx, const void* w, int rank, int T, int N, int D, const float* bias,
-                      const float* a_log, float inv_tau, cudaStream_t stream);
+                      const float* a_log, float inv_tau, int early_weights, cudaStream_t stream);
 int zi_unit_norm(float* x, int ld, int T, int heads, int d, float eps, float scale, cudaStream_t stream);
 int zi_sigmoid_rows(float* out, int ldo, const void* x, int ldx, int dtype, int rows, int W, cudaStream_t stream);
 int zi_linear_recurrence(float* out, int ldo, const void* q, int ldq, const void* k, int ldk, int qk_dtype, const void* v,

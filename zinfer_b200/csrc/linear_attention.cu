@@ -100,14 +100,16 @@ __global__ void decay_kernel(float* __restrict__ z, size_t total, int N, int D, 
 template <int R>
 __global__ void __launch_bounds__(256)
 low_rank_decay_kernel(float* __restrict__ out, const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ w, int rank,
-                      int T, int N, int D, int tokens, const float* __restrict__ bias, const float* __restrict__ a_log, float inv_tau) {
+                      int T, int N, int D, int tokens, const float* __restrict__ bias, const float* __restrict__ a_log, float inv_tau,
+                      int early) {
   pdl_launch_dependents();
   const int c = blockIdx.x * blockDim.x + threadIdx.x, t0 = blockIdx.y * tokens;
-  pdl_wait();
+  if (!early) pdl_wait();                            // early: no kernel of this step writes the weights
   float wr[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) wr[r] = c < N && r < rank ? to_f32(w[(size_t)c * rank + r]) : 0.f;
   const float add = c < N && bias ? bias[c] : 0.f, rate = c < N && a_log ? expf(a_log[c / D]) : 0.f;
+  if (early) pdl_wait();
   if (c >= N) return;
   const int t1 = min(T, t0 + tokens);
   for (int t = t0; t < t1; ++t) {
@@ -806,14 +808,14 @@ extern "C" int zi_decay(float* z, long long rows, int N, int D, const float* bia
 
 // Mode as for zi_decay: with a_log the softplus form, without it the root of a sigmoid.
 extern "C" int zi_low_rank_decay(float* out, const void* x, int ldx, const void* w, int rank, int T, int N, int D, const float* bias,
-                                 const float* a_log, float inv_tau, cudaStream_t stream) {
+                                 const float* a_log, float inv_tau, int early_weights, cudaStream_t stream) {
   if (T <= 0 || N <= 0) return 0;
   if (rank <= 0 || rank > 32) return zi_refuse("low_rank_decay: rank %d is outside 1..32", rank);
   if (D <= 0 || T > 65535 * 8) return zi_refuse("low_rank_decay: %d tokens, heads of %d", T, D);
   const int tokens = T <= 64 ? 1 : 8;
   const dim3 grid((N + 255) / 256, (T + tokens - 1) / tokens);
   zi_launch(rank <= 16 ? low_rank_decay_kernel<16> : low_rank_decay_kernel<32>, grid, dim3(256), 0, stream, out, (const __nv_bfloat16*)x, ldx,
-            (const __nv_bfloat16*)w, rank, T, N, D, tokens, bias, a_log, inv_tau);
+            (const __nv_bfloat16*)w, rank, T, N, D, tokens, bias, a_log, inv_tau, early_weights);
   return zi_check_launch("low_rank_decay");
 }
 

@@ -1845,10 +1845,11 @@ def decay_exp_softplus_(z: torch.Tensor, bias: Optional[torch.Tensor], a_log: to
 
 
 def low_rank_decay(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], a_log: Optional[torch.Tensor], tau: float,
-                   head_dim: int) -> torch.Tensor:
+                   head_dim: int, fresh_weights: bool = True) -> torch.Tensor:
     """float32 decays [T, N] of ``z = x [T, rank] @ w [N, rank]^T``: with ``a_log`` as :func:`decay_exp_softplus_`, else as
     :func:`decay_sigmoid_root_` has them.  One kernel for bfloat16 operands of a rank up to 32; otherwise the product and the
-    decay's kernel."""
+    decay's kernel.  ``fresh_weights`` False: no kernel of this step writes ``w``, ``bias`` or ``a_log``, which may then be read
+    before the wait for the kernels before this one."""
     T, rank = x.shape
     N = w.shape[0]
     if not (x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and rank <= 32 and x.stride(1) == 1 and w.is_contiguous()
@@ -1862,7 +1863,7 @@ def low_rank_decay(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor
     out = torch.empty((T, N), dtype=torch.float32, device=x.device)
     with _prof.region("decay (low-rank product)", lambda: _nb(out, w) + T * rank * 2, 2 * T * N * rank):
         _check(lib().zi_low_rank_decay(_ptr(out), _ptr(x), x.stride(0), _ptr(w), rank, T, N, head_dim, _ptr(bias), _ptr(a_log),
-                                       ctypes.c_float(1.0 / tau), _stream()), "low_rank_decay")
+                                       ctypes.c_float(1.0 / tau), 0 if fresh_weights else 1, _stream()), "low_rank_decay")
     return out
 
 

@@ -85,7 +85,7 @@ class GatedLinearAttention(Mixer):
         qk, hv = self.heads * self.dim, self.heads * self.vdim
         proj = ops.linear(x, self.w_in, out_dtype=self.ctx.dtype, fresh_weight=False)
         q, k, v, g = proj[:, :qk], proj[:, qk:2 * qk], proj[:, 2 * qk:2 * qk + hv], proj[:, 2 * qk + hv:2 * qk + 2 * hv]
-        decay = ops.low_rank_decay(proj[:, 2 * qk + 2 * hv:], self.w_a2, self.a_bias, None, self.tau, self.dim)
+        decay = ops.low_rank_decay(proj[:, 2 * qk + 2 * hv:], self.w_a2, self.a_bias, None, self.tau, self.dim, fresh_weights=False)
         o = ops.channel_decay_recurrence(q, k, v, decay, None, self.dim ** -0.5, cache.state, self.heads, self.heads, self.dim, self.vdim, step,
                                          fast=self.ctx.dtype == torch.bfloat16)
         y = ops.head_norm_gate(o, self.norm, self.eps, g, "silu", self.heads, self.vdim, self.ctx.dtype)
@@ -235,7 +235,7 @@ class GatedDeltaRule(Mixer):
         ops.unit_norm_(qkv[:, :2 * qk], 2 * self.kv_heads, self.dim, self.UNIT_EPS)      # q's heads, then k's
         beta = ops.sigmoid_rows(proj[:, C:C + H])
         a0 = C + H
-        decay = ops.low_rank_decay(proj[:, a0:a0 + self.decay_rank], self.w_a2, self.dt_bias, self.a_log, 1.0, self.dim)
+        decay = ops.low_rank_decay(proj[:, a0:a0 + self.decay_rank], self.w_a2, self.dt_bias, self.a_log, 1.0, self.dim, fresh_weights=False)
         o = ops.channel_decay_recurrence(q, k, v, decay, beta, self.dim ** -0.5, s_view, H, self.kv_heads, self.dim, self.vdim, step,
                                          fast=self.ctx.dtype == torch.bfloat16)
         gate = ops.linear(proj[:, a0 + self.decay_rank:], self.w_g2, out_dtype=self.ctx.dtype, fresh_weight=False)

@@ -48,8 +48,11 @@ class SwiGLUMLP(FeedForward):
         self.w_down = tensors[self.names[2]].contiguous()
 
     def forward(self, x):
-        if self.interleaved:
+        if self.interleaved and self.ctx.dtype == torch.bfloat16:
             act = ops.linear_swiglu(x, self.w_gate_up, out_dtype=self.ctx.dtype, activation=self.activation)
+        elif self.interleaved:       # 32-bit products have no gate of their own
+            gu = ops.linear(x, self.w_gate_up, out_dtype=self.ctx.dtype, fresh_weight=False)
+            act = ops.swiglu(gu, out_dtype=self.ctx.dtype, interleave=ops.SWIGLU_INTERLEAVE, activation=self.activation)
         else:
             gu = ops.linear(x, self.w_gate_up, out_dtype=self.ctx.dtype, allow_partials=True, fresh_weight=False)
             if self.clamped:
