@@ -181,7 +181,8 @@ paged_attention_kernel(T* __restrict__ out, int out_stride, const T* __restrict_
 // the same order, one chain over a tile's keys), so both give the same bits.
 // Bound by shared-memory reads in prompts and by the chain of a tile's steps for single tokens.  Measured, 16 heads of 64
 // over 4 kv heads: prompts of 354 and 158 tokens 281 -> 101 us, 12 requests with prompts of 46 to 134 tokens through
-// prompts and 24 decoded tokens each 113 -> 23 us a launch.
+// prompts and 24 decoded tokens each 113 -> 23 us a launch.  A short prompt of one request has a quarter of the plain kernel's
+// blocks and gains all the same: 16 tokens 21 -> 13 us, 64 tokens 47 -> 21.
 template <int D, int HG>
 struct F32Attention {
   static constexpr int ROWS = BQ * HG, KP = D + 4, SP = BK + 4;         // pitches: rows four banks apart

@@ -31,9 +31,10 @@
 // that bring one token are left alone and have no place.
 //
 // Measured, 2,048 tokens, 8 heads of 128 x 256 (the walk token by token -> chunks): plain form with bfloat16 q, k, v 756 -> 182 us,
-// delta rule 833 -> 259 us.  Relative errors of outputs and states against 64 bits, 1e-7 (the walk -> chunks): plain 4.9, 5.8 ->
-// 3.3, 3.6, delta rule 2.1, 1.4 -> 1.6, 0.9.  (Two tf32 parts, 22 bits, and rows that took off their terms one by one: 168 and 242 us,
-// but 2.5, 1.7 with the delta rule, and plain at 8 x 64 tokens 1.65 against the walk's 1.52.)
+// delta rule 833 -> 259 us; one kernel at a time the scores 39 and 48 us, the triangular systems 47, the walk 140 and 185.
+// Relative errors of outputs and states against 64 bits, 1e-7 (the walk -> chunks): plain 4.9, 5.8 -> 3.3, 3.6, delta rule
+// 2.1, 1.4 -> 1.6, 0.9.  (Two tf32 parts, 22 bits, and rows that took off their terms one by one: 168 and 242 us, but 2.5, 1.7
+// with the delta rule, and plain at 8 x 64 tokens 1.65 against the walk's 1.52.)
 #include "api.h"
 #include "common.cuh"
 

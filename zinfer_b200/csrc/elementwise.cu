@@ -1308,8 +1308,9 @@ norm_residual_vec_kernel(float* __restrict__ h, const TA* __restrict__ a, float 
   }
 }
 
-// Few rows (a decode step): a row's loads are spread over up to 1024 threads, four columns of a thread in flight
-// together, and the summed update is kept in shared memory so that partial sums are read once.
+// Rows of any width and alignment, and more than 512 rows whose updates are partial sums: a row's loads are spread over up to
+// 1024 threads, four columns of a thread in flight together, and the summed update is kept in shared memory so that partial
+// sums are read once.
 template <typename TA, typename TB, typename TO>
 __global__ void __launch_bounds__(1024)
 norm_residual_kernel(float* __restrict__ h, const TA* __restrict__ a, const float* __restrict__ ap, int as, size_t az, float sa,

@@ -82,8 +82,8 @@ __device__ __forceinline__ void f32_chunk(float (&acc)[TM][TN], const float* xs,
   }
 }
 
-// A chunk's pieces (all PIECES of it, or fewer at the end of K) in turn, each read one ahead of its use (512 x 6144 x 1024 195 ->
-// 187 us; with the ring of the kernel for few rows 189, and 512 x 1024 x 3072 125 instead of 120).
+// The same for the larger tiles, each piece read one ahead of its use (512 x 6144 x 1024 195 -> 187 us; with the ring above 189,
+// and 512 x 1024 x 3072 125 instead of 120).
 template <int TM, int TN, int GAP_A, int GAP_B, int PIECES, int UNROLL>
 __device__ __forceinline__ void f32_chunk_pairs(float (&acc)[TM][TN], const float* xs, const float* ws, int pieces) {
   F32Piece<TM, TN> even, odd;
@@ -106,8 +106,8 @@ __device__ __forceinline__ void f32_chunk_pairs(float (&acc)[TM][TN], const floa
 
 // Bound by shared memory: a 16-byte read by a warp takes four of the SM's 128-byte clocks whatever the addresses, so the
 // plain kernel's one-word reads left the multiply-adds idle most of the time (512 x 6144 x 1024: 336 us, 19 TFLOP/s; now
-// 187 us, 34, of the 69 that independent chains of fmaf reach here).  A ring of STAGES chunks of KC columns, filled by cp.async; a thread owns TM x TN outputs, rows BM / TM and columns
-// BN / TN apart, and reads both operands as 16-byte pieces along k.  `early`: w is not written by a kernel of this
+// 187 us, 34, of the 69 that independent chains of fmaf reach here).  A ring of STAGES chunks of KC columns, filled by
+// cp.async; a thread owns TM x TN outputs, rows BM / TM and columns BN / TN apart, and reads both operands as 16-byte pieces along k.  `early`: w is not written by a kernel of this
 // step, so its first chunks are requested before the wait for the kernels before this one.
 template <typename T, typename TO>
 __global__ void __launch_bounds__(T::THREADS)
@@ -186,11 +186,12 @@ int launch_f32_tile(void* out, const float* x, const float* w, int M, int N, int
 }
 
 // ---------------------------------------------------------------------------------------------- few rows
-// Up to 32 rows: the same tiles with a warp of their own for the copies.  One lane per operand row asks for KC columns of
-// it in one untiled bulk copy (both ends on 16-byte boundaries, sizes of whole 16 bytes: K % 4 == 0), so the warps that
-// multiply issue nothing but shared-memory reads and multiply-adds.  Bound by the chain itself: K dependent multiply-adds of
-// four clocks and the reads that feed them (12 x 1024 x 1024: 8.5 us, 4 MB of weights; 9.5 with pieces read one ahead; 18 us with copies by the same warps,
-// whose addresses cost more issue slots than the product).  One tensor copy a chunk in the place of one bulk copy a row,
+// Up to 32 rows, and more where 32 x 32 tiles would not make a block for every SM: the same tiles with a warp of their own
+// for the copies.  One lane per operand row asks for KC columns of it in one untiled bulk copy (both ends on 16-byte
+// boundaries, sizes of whole 16 bytes: K % 4 == 0), so the warps that multiply issue nothing but shared-memory reads and
+// multiply-adds.  Bound by the chain itself: K dependent multiply-adds of four clocks and the reads that feed them (12 x 1024
+// x 1024: 8.5 us, 4 MB of weights; 9.5 with pieces read one ahead; 18 us with copies by the same warps, whose addresses
+// cost more issue slots than the product).  One tensor copy a chunk in the place of one bulk copy a row,
 // its lines swizzled, was measured too: 11.1 us, for the addresses of the swizzled reads.
 template <int BM_, int BN_, int TM_, int TN_, int KC_, int STAGES_, int AHEAD_>
 struct F32Few {

@@ -782,7 +782,8 @@ static void plan_single(int M, int N, int K, int sm_count, int* plan) {
   }
   if (!swap && sm_count > 0 && 2 * tiles <= sm_count) {
     // A few hundred tokens: the tiles leave most SMs idle, and a CTA walks all of K at the pace
-    // of its own copies (about 0.45 us a k-block).  Splitting K spreads the walk over more CTAs
+    // of its own copies (about 0.45 us a k-block when this was measured; 0.25 to 0.37 since the copies are issued by an
+    // elected lane, so that splits now begin somewhat too early).  Splitting K spreads the walk over more CTAs
     // until L2 cannot feed them (about 10 TB/s), and costs the partial sums' round trip through
     // memory and a kernel to add them (about 8 us in all, measured at 256 to 512 tokens).  Split when
     // that model promises a tenth or more (512 tokens x 4096 x 12288: 78 us whole, 61 us in two).

@@ -37,9 +37,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
 }
 // A warp's number in a register that the compiler knows to be the same in all its lanes, and one lane of a whole warp.
 // The instructions that issue copies and products take their operands from registers shared by the warp.  Issued from a
-// branch that one lane takes (`if (lane == 0)`), the compiler cannot know them shared and moves each by a loop over the
-// lanes: four MMAs of a k-block took 0.34 us whatever their size and two copies 0.28, a whole k-block 0.44 us; with the
-// whole warp in the loop and elect.sync around the issue alone 0.21 .. 0.29, 0.20 .. 0.27 and 0.29 .. 0.32 us.
+// branch that one lane takes (`if (lane == 0)`), four MMAs of a k-block took 0.34 us whatever their size and two copies
+// 0.28, a whole k-block 0.44 us; with the whole warp in the loop and elect.sync around the issue alone 0.18 .. 0.29,
+// 0.16 .. 0.26 and 0.23 .. 0.29 us by the tile's size.
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
