@@ -255,7 +255,7 @@ gemm_f32_few_kernel(TO* __restrict__ out, const float* __restrict__ x, const flo
       copy_x(c);
     }
     for (int c = ahead; c < chunks; ++c) {
-      if (!mbar_wait(&empty[c % STAGES], ((c / STAGES) & 1) ^ 1)) {     // a lane that gives up leaves; __syncwarp counts those that stay
+      if (!warp_mbar_wait(&empty[c % STAGES], ((c / STAGES) & 1) ^ 1)) {
         failed = true;
         break;
       }
@@ -279,7 +279,9 @@ gemm_f32_few_kernel(TO* __restrict__ out, const float* __restrict__ x, const flo
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
   for (int c = 0; c < chunks; ++c) {
     const int s = c % STAGES;
-    if (!mbar_wait(&full[s], (c / STAGES) & 1)) {
+    // (one answer for the warp, here and above: 12 requests' generation 28.8 ms; 28.6 with each lane on its own, and 28.8 again with
+    // a note that the lane keeps or the vote behind the chunk)
+    if (!warp_mbar_wait(&full[s], (c / STAGES) & 1)) {
       failed = true;
       break;
     }
